@@ -28,7 +28,8 @@ struct shwfs_screen {
   float* scr = nullptr;           // ny x nx, physical order
   double* a[2] = {nullptr, nullptr};  // [0] columns: ny x 2ny; [1] rows: nx x 2nx
   double* b[2] = {nullptr, nullptr};  // [0] ny x ny; [1] nx x nx
-  double* noise = nullptr;        // max(ny, nx)
+  double* noise = nullptr;        // max(ny, nx): injected normals of one line
+  int numSMs = 1;
   shwfs::PhiloxKeys keys{};
   unsigned long long added = 0;   // extrusions so far (the noise stream's frame index)
   cudaStream_t stream = nullptr;
@@ -38,65 +39,147 @@ namespace shwfs {
 
 namespace {
 
-constexpr int kScrWarps = 8;
-
-// standard normals for one extrusion: element j from the stream of
-// (seed, extrusion, j, purpose 3)
-__global__ void screen_noise_kernel(PhiloxKeys keys, unsigned long long ext, int n, double* out) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    KeyedStream st(keys, ext, j, 0, 3);
-    out[j] = (double)normal_counter(st);
-  }
+// (double)x by integer operations for zeros and normal values: the
+// conversion instruction runs on the FP64 pipe, which the kernels below are
+// bound by
+__device__ __forceinline__ double to_double(float x) {
+  const uint32_t u = __float_as_uint(x), m = u & 0x7fffffffu;
+  if (m - 1u < 0x007fffffu || m >= 0x7f800000u) return (double)x;  // subnormal, infinite or NaN
+  const uint32_t hi = (u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u);
+  return __hiloint2double((int)hi, (int)(u << 29));
 }
 
-// one new column (axis 0) or row (axis 1): warp per output element
-__global__ void screen_extrude_kernel(float* __restrict__ scr, int ny, int nx, int rs, int cs, int axis, int start,
-                                      const double* __restrict__ A, const double* __restrict__ B,
-                                      const double* __restrict__ noise, double coeff, double step) {
+// One new line (axis 0 a column, 1 a row): kLineThreads threads per output
+// element, rowsPerCta elements per CTA, so that about one CTA per SM covers
+// the line.  Bound by reading A and B once (24 len^2 bytes, L2-resident
+// between lines) and by the FP64 rate (3 len^2 multiply-adds at about two a
+// cycle and SM: 2.6 us for 741 elements); a warp per element with its z
+// gathered by modulo from the circular buffer took 35 us for 741.  Here a
+// thread has all its 18 matrix elements of a chunk in flight before the
+// vectors are staged in shared memory, and the line's normals, B n and the
+// matrix loads, which do not depend on the line before, run ahead of
+// griddepcontrol.wait: successive lines are launched programmatically and
+// overlap in that part.
+constexpr int kLineThreads = 64;  // per output element
+constexpr int kLineUnroll = 12;     // elements of each of A's two blocks and of B per thread and chunk
+constexpr int kLineChunk = kLineThreads * kLineUnroll;
+constexpr int kLineMaxRows = 8;
+
+__global__ void __launch_bounds__(kLineThreads* kLineMaxRows)
+    screen_line_kernel(float* __restrict__ scr, int ny, int nx, int rs, int cs, int axis, int start,
+                       const double* __restrict__ A, const double* __restrict__ B, const PhiloxKeys keys,
+                       unsigned long long ext, const double* __restrict__ noise, double coeff, double step) {
+  __shared__ double s_n[kLineChunk], s_z[2][kLineChunk];
+  __shared__ double s_red[kLineThreads * kLineMaxRows];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int len = axis == 0 ? ny : nx;  // output length; Z has 2 len entries
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * kScrWarps + (threadIdx.x >> 5);
-  if (i >= len) return;
-  // logical element k of line l of A's block l: at the end, 0 the older of
-  // the last two lines and 1 the last; at the start, 0 the second line and
-  // 1 the first (the edge)
-  auto z = [&](int l, int k) {
-    if (axis == 0) {
-      const int x = start ? 1 - l : nx - 2 + l;
-      return (double)scr[(long long)((rs + k) % ny) * nx + (cs + x) % nx];
-    }
-    const int y = start ? 1 - l : ny - 2 + l;
-    return (double)scr[(long long)((rs + y) % ny) * nx + (cs + k) % nx];
-  };
-  const double* ar = A + (long long)i * 2 * len;
-  const double* br = B + (long long)i * len;
-  double az = 0.0, bn = 0.0;
-  for (int j = lane; j < 2 * len; j += 32) az += ar[j] * z(j / len, j % len);
-  for (int j = lane; j < len; j += 32) bn += br[j] * noise[j];
+  const int tid = threadIdx.x, t = tid & (kLineThreads - 1), g = tid / kLineThreads;
+  const int rows = blockDim.x / kLineThreads;
+  const int i = blockIdx.x * rows + g;
+  const bool live = i < len;
+  const double* ar = A + (long long)(live ? i : 0) * 2 * len;
+  const double* br = B + (long long)(live ? i : 0) * len;
+  // physical position of line l of A's block l: at the end, 0 the older of
+  // the last two lines and 1 the last; at the start, 0 the second line and 1
+  // the first (the edge)
+  int line[2];
+  const int lines = axis == 0 ? nx : ny, origin = axis == 0 ? cs : rs, along = axis == 0 ? rs : cs;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    az += __shfl_xor_sync(0xffffffffu, az, o);
-    bn += __shfl_xor_sync(0xffffffffu, bn, o);
+  for (int l = 0; l < 2; l++) {
+    line[l] = origin + (start ? 1 - l : lines - 2 + l);
+    if (line[l] >= lines) line[l] -= lines;
   }
-  if (lane == 0) {
-    const double v = az + bn * coeff + step;
-    // the new line replaces the one dropped: at the end the first line
-    // (physical column cs, row rs), at the start the last
-    const int pc = start ? (cs + nx - 1) % nx : cs, pr = start ? (rs + ny - 1) % ny : rs;
-    if (axis == 0)
-      scr[(long long)((rs + i) % ny) * nx + pc] = (float)v;
-    else
-      scr[(long long)pr * nx + (cs + i) % nx] = (float)v;
+  double az = 0.0, bn = 0.0;
+  for (int j0 = 0; j0 < len; j0 += kLineChunk) {
+    const int cnt = min(kLineChunk, len - j0);
+    double a0[kLineUnroll], a1[kLineUnroll], b[kLineUnroll];
+#pragma unroll
+    for (int u = 0; u < kLineUnroll; u++) {
+      const int j = t + u * kLineThreads;
+      const bool in = live && j < cnt;
+      b[u] = in ? br[j0 + j] : 0.0;
+      a0[u] = in ? ar[j0 + j] : 0.0;
+      a1[u] = in ? ar[len + j0 + j] : 0.0;
+    }
+    if (j0) __syncthreads();  // the previous chunk's vectors are consumed
+    // standard normals of this extrusion: element j from the stream of
+    // (seed, extrusion, j, purpose 3)
+    for (int j = tid; j < cnt; j += blockDim.x) {
+      if (noise) {
+        s_n[j] = noise[j0 + j];
+      } else {
+        KeyedStream st(keys, ext, j0 + j, 0, 3);
+        s_n[j] = to_double(normal_counter(st));
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kLineUnroll; u++) {
+      const int j = t + u * kLineThreads;
+      if (j < cnt) bn = fma(b[u], s_n[j], bn);
+    }
+    // the lines before this one are complete and visible from here on
+    if (j0 == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int j = tid; j < cnt; j += blockDim.x) {
+      int k = along + j0 + j;
+      if (k >= len) k -= len;
+#pragma unroll
+      for (int l = 0; l < 2; l++)
+        s_z[l][j] = to_double(axis == 0 ? scr[(long long)k * nx + line[l]] : scr[(long long)line[l] * nx + k]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kLineUnroll; u++) {
+      const int j = t + u * kLineThreads;
+      if (j < cnt) {
+        az = fma(a0[u], s_z[0][j], az);
+        az = fma(a1[u], s_z[1][j], az);
+      }
+    }
+  }
+  s_red[tid] = fma(bn, coeff, az);
+  __syncthreads();
+  // one warp per element sums its threads' parts
+  const int w = tid >> 5, lane = tid & 31, io = blockIdx.x * rows + w;
+  if (w < rows && io < len) {
+    double v = 0.0;
+#pragma unroll
+    for (int k = 0; k < kLineThreads / 32; k++) v += s_red[w * kLineThreads + k * 32 + lane];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) {
+      // the new line replaces the one dropped: at the end the first line
+      // (physical column cs, row rs), at the start the last
+      int pl = start ? origin - 1 : origin, k = along + io;
+      if (pl < 0) pl += lines;
+      if (k >= len) k -= len;
+      scr[axis == 0 ? (long long)k * nx + pl : (long long)pl * nx + k] = (float)(v + step);
+    }
   }
 }
 
-__global__ void screen_window_kernel(const float* __restrict__ scr, int ny, int nx, int rs, int cs, int y0, int x0,
-                                     int h, int w, float* __restrict__ out, long long stride) {
-  const long long total = (long long)h * w;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total;
-       k += (long long)gridDim.x * blockDim.x) {
-    const int y = (int)(k / w), x = (int)(k - (long long)y * w);
-    out[(long long)y * stride + x] = scr[(long long)((rs + y0 + y) % ny) * nx + (cs + x0 + x) % nx];
+// an h x w window, a block per row, with the circular wraps by comparison (a
+// 64-bit division and two modulo operations per pixel took 6 us for
+// 740 x 740 against 1 us of copy time); launched programmatically behind the
+// line kernels
+constexpr int kWinThreads = 256;
+__global__ void __launch_bounds__(kWinThreads)
+    screen_window_kernel(const float* scr, int ny, int nx, int rs, int cs, int y0, int x0, int h, int w,
+                         float* __restrict__ out, long long stride) {
+  int px0 = cs + x0;  // physical column of the window's first
+  if (px0 >= nx) px0 -= nx;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (int y = blockIdx.x; y < h; y += gridDim.x) {
+    int py = rs + y0 + y;
+    if (py >= ny) py -= ny;
+    const float* src = scr + (long long)py * nx;
+    float* dst = out + y * stride;
+#pragma unroll 4
+    for (int x = threadIdx.x; x < w; x += kWinThreads) {
+      int px = px0 + x;
+      if (px >= nx) px -= nx;
+      dst[x] = src[px];
+    }
   }
 }
 
@@ -229,7 +312,10 @@ shwfs_status shwfs_screen_create(int ny, int nx, const float* init, const double
     shwfs::set_philox_keys(tmp);
     s->keys = tmp.philoxKeys;
   }
-  cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&s->numSMs, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = upload(&s->scr, init, (size_t)ny * nx);
   if (e == cudaSuccess && ay) e = upload(&s->a[0], ay, (size_t)ny * 2 * ny);
   if (e == cudaSuccess && by) e = upload(&s->b[0], by, (size_t)ny * ny);
@@ -252,24 +338,34 @@ shwfs_status shwfs_screen_add(shwfs_screen* s, int axis, int n, double coeff_tur
   if (!s->a[axis]) return engine_fail(SHWFS_ERR_INVALID, "screen_add: no matrices for this axis");
   cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
   const int len = axis == 0 ? s->ny : s->nx;
+  // elements per CTA: about one CTA per SM (more for lines of over eight
+  // elements per SM)
+  const int rows = std::max(1, std::min(shwfs::kLineMaxRows, (len + s->numSMs - 1) / s->numSMs));
   for (int k = 0; k < n; k++) {
-    if (noise) {
+    if (noise)
       SCK(cudaMemcpyAsync(s->noise, noise + (size_t)k * len, len * sizeof(double), cudaMemcpyHostToDevice, st),
           "screen_add noise");
-    } else {
-      shwfs::screen_noise_kernel<<<(len + 255) / 256, 256, 0, st>>>(s->keys, s->added, len, s->noise);
-      SCK(cudaGetLastError(), "screen_noise_kernel");
-    }
-    const int blocks = (len + shwfs::kScrWarps - 1) / shwfs::kScrWarps;
-    shwfs::screen_extrude_kernel<<<blocks, shwfs::kScrWarps * 32, 0, st>>>(
-        s->scr, s->ny, s->nx, s->rs, s->cs, axis, start, s->a[axis], s->b[axis], s->noise, coeff_turb,
-        k == 0 ? step : 0.0);
-    SCK(cudaGetLastError(), "screen_extrude_kernel");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((len + rows - 1) / rows));
+    cfg.blockDim = dim3((unsigned)(rows * shwfs::kLineThreads));
+    cfg.stream = st;
+    // programmatic launch: injected normals are read ahead of the kernel's
+    // wait, so a line that takes them is launched in plain stream order
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = noise ? 0 : 1;
+    const double* injected = noise ? s->noise : nullptr;
+    SCK(cudaLaunchKernelEx(&cfg, shwfs::screen_line_kernel, s->scr, s->ny, s->nx, s->rs, s->cs, axis, start,
+                           (const double*)s->a[axis], (const double*)s->b[axis], s->keys, s->added, injected,
+                           coeff_turb, k == 0 ? step : 0.0),
+        "screen_line_kernel");
     if (axis == 0)
       s->cs = start ? (s->cs + s->nx - 1) % s->nx : (s->cs + 1) % s->nx;
     else
       s->rs = start ? (s->rs + s->ny - 1) % s->ny : (s->rs + 1) % s->ny;
-    s->added++;  // the next extrusion's noise overwrites s->noise in stream order
+    s->added++;  // the next extrusion's injected noise overwrites s->noise in stream order
   }
   if (!stream) SCK(cudaStreamSynchronize(st), "screen_add sync");
   return SHWFS_OK;
@@ -280,11 +376,18 @@ shwfs_status shwfs_screen_window(shwfs_screen* s, int y0, int x0, int h, int w, 
   if (!s || !out || y0 < 0 || x0 < 0 || h < 1 || w < 1 || y0 + h > s->ny || x0 + w > s->nx || out_stride < w)
     return engine_fail(SHWFS_ERR_INVALID, "screen_window: window outside the screen");
   cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
-  const long long total = (long long)h * w;
-  const int blocks = (int)std::min<long long>((total + 255) / 256, 152LL * 8);
-  shwfs::screen_window_kernel<<<blocks, 256, 0, st>>>(s->scr, s->ny, s->nx, s->rs, s->cs, y0, x0, h, w, out,
-                                                       (long long)out_stride);
-  SCK(cudaGetLastError(), "screen_window_kernel");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min(h, s->numSMs * 8));
+  cfg.blockDim = dim3(shwfs::kWinThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  SCK(cudaLaunchKernelEx(&cfg, shwfs::screen_window_kernel, (const float*)s->scr, s->ny, s->nx, s->rs, s->cs, y0, x0, h, w,
+                         out, (long long)out_stride),
+      "screen_window_kernel");
   if (!stream) SCK(cudaStreamSynchronize(st), "screen_window sync");
   return SHWFS_OK;
 }

@@ -1096,12 +1096,12 @@ shwfs_status enqueue_slope(shwfs_handle* h, cudaStream_t st) {
   float* cents = h->cents.on_device ? (float*)h->cents.data : (h->centsDirect ? h->centsMapped : h->d_cents.p);
   float* bimg = h->bimg.on_device ? (float*)h->bimg.data : (h->bimgDirect ? h->bimgMapped : h->d_bimg.p);
   const int mm = h->nimg * h->nimg;
+  bool didUnlit = false;
   if (!h->lit.empty()) {
     WfsArgs a = make_args(h, nullptr, cents, bimg, 1, 0, kPost);
-    a.TS = std::max(1, std::min(64, 4096 / mm));
-    CK(launch_image(a, img, h->imageDims, h->imageCols, h->d_subapLoc.p, h->numSMs, st));
+    CK(launch_image(a, img, h->imageDims, h->imageCols, h->d_subapLoc.p, h->numSMs, st, &didUnlit));
   }
-  if (!h->unlit.empty()) {
+  if (!h->unlit.empty() && !didUnlit) {
     WfsArgs a = make_args(h, nullptr, cents, bimg, 1, 0, 0);
     if (h->noiseMode == SHWFS_NOISE_REFERENCE && h->imageOnly) {
       RefNoiseArgs r{};

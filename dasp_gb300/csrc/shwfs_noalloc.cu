@@ -140,7 +140,6 @@ extern "C" shwfs_status shwfs_image_centroids_noalloc(const shwfs_image_job* job
   a.m = m;
   a.ncen = job->ncen;
   a.nframes = 1;
-  a.TS = m * m <= 4096 ? (4096 / (m * m) < 64 ? 4096 / (m * m) : 64) : 1;
   a.floorv = job->noiseFloor;
   a.threshType = job->threshType;
   a.calsource = job->calsource;

@@ -825,9 +825,11 @@ cudaError_t launch_sample_noise(const float* lam, long long n, unsigned long lon
                                 int kind, float* out, cudaStream_t stream);
 // store v in one device counter, in stream order
 cudaError_t launch_set_counter(unsigned long long* ctr, unsigned long long v, cudaStream_t stream);
-// image-input (runSlope) kernel over the lit subapertures (wfs_image.cu)
+// image-input (runSlope) kernel over the lit subapertures (wfs_image.cu);
+// didUnlit (optional) receives whether it also zeroed the centroids of the
+// unlit subapertures of a.unlit
 cudaError_t launch_image(const WfsArgs& a, const float* img, int dims, int npxlx, const int* loc, int numSMs,
-                         cudaStream_t stream);
+                         cudaStream_t stream, bool* didUnlit = nullptr);
 // copy the listed subapertures' images src -> dst (dst: mapped host memory)
 cudaError_t launch_publish(const float* src, float* dst, const int* list, int n, int mm, cudaStream_t stream);
 // physical integration: acc = (first ? sub : acc + sub), then acc *= scale

@@ -202,8 +202,70 @@ __device__ __forceinline__ void centroid_tile(const WfsArgs& a, int ns, const in
     const int tid = threadIdx.x;
     const int m = a.m, mm = m * m;
     // ---- 9: centroids, calibration, reference subtraction ----
-    const bool seqMode = a.opticalBinning == 1 || a.fitSize != 0 || a.gaussianFit > 0 || a.cob != 0;
-    if (seqMode) {
+    const bool seqMode = a.opticalBinning == 1 || a.fitSize != 0 || a.gaussianFit > 0 || (a.cob != 0 && a.cob != 1);
+    if (!seqMode && a.cob == 1) {
+      // CoG in the ncen x ncen window about the brightest pixel (its first
+      // occurrence; pixel 0 when none is positive): one warp per subaperture
+      // (one thread scanned the image and then the window: about 4 us of a
+      // 20 x 20 correlation image's tile)
+      const int warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+      const int n = m, ncen = a.ncen;
+      for (int s = warp; s < ns; s += nwarps) {
+        const float* img = img_of(s);
+        const int i = s_subap[s];
+        float mx = 0.f;
+        int mpos = 0x7fffffff;
+        for (int k = lane; k < mm; k += 32)
+          if (img[k] > mx) {
+            mx = img[k];
+            mpos = k;
+          }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+          const float v = __shfl_xor_sync(0xffffffffu, mx, o);
+          const int q = __shfl_xor_sync(0xffffffffu, mpos, o);
+          if (v > mx || (v == mx && q < mpos)) {
+            mx = v;
+            mpos = q;
+          }
+        }
+        if (mpos == 0x7fffffff) mpos = 0;
+        int sy = mpos / n, sx = mpos - sy * n;
+        sx = (int)((float)sx - 0.5f * (float)ncen + 0.5f);  // exact in float
+        sy = (int)((float)sy - 0.5f * (float)ncen + 0.5f);
+        sx = max(0, min(sx, n - ncen));
+        sy = max(0, min(sy, n - ncen));
+        const float* wt = a.centWeightDim == 2 ? s_cw
+                          : (a.centWeightDim == 4 ? a.centWeight + (long long)i * mm : nullptr);
+        const float inv_nc = 1.0f / (float)ncen;
+        float sum = 0.f, cx = 0.f, cy = 0.f;
+        for (int k = lane; k < ncen * ncen; k += 32) {
+          const int rr = div_small(k, ncen, inv_nc);
+          const int r = sy + rr, c = sx + (k - rr * ncen);
+          const float t = wt ? img[r * n + c] * wt[r * n + c] : img[r * n + c];
+          sum += t;
+          cx += t * c;
+          cy += t * r;
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+          sum += __shfl_xor_sync(0xffffffffu, sum, o);
+          cx += __shfl_xor_sync(0xffffffffu, cx, o);
+          cy += __shfl_xor_sync(0xffffffffu, cy, o);
+        }
+        if (lane == 0) {
+          if (sum > 0) {
+            cx = cx / sum + sx;
+            cy = cy / sum + sy;
+            cx -= 0.5f * (float)(n - 1);
+            cy -= 0.5f * (float)(n - 1);
+          } else {
+            cx = cy = 0.f;
+          }
+          calibrate_and_store(a, i, s_frame[s], cx, cy);
+        }
+      }
+    } else if (seqMode) {
       for (int s = tid; s < ns; s += blockDim.x) {
         float* img = img_of(s);
         const int i = s_subap[s];
@@ -225,25 +287,17 @@ __device__ __forceinline__ void centroid_tile(const WfsArgs& a, int ns, const in
           const int n = m, ncen = a.ncen;
           float mx = 0.f;
           int mpos = 0;
-          if (a.cob == 1) {
-            for (int k = 0; k < n * n; k++)
-              if (img[k] > mx) {
-                mx = img[k];
-                mpos = k;
-              }
-          } else {
-            for (int k = 0; k < n * n; k++)
-              if (img[k] < mx || mx == 0) {
-                mx = img[k];
-                mpos = k;
-              }
-          }
+          for (int k = 0; k < n * n; k++)
+            if (img[k] < mx || mx == 0) {
+              mx = img[k];
+              mpos = k;
+            }
           int sx = (int)(mpos % n - ncen / 2. + 0.5), sy = (int)(mpos / n - ncen / 2. + 0.5);
           sx = max(0, min(sx, n - ncen));
           sy = max(0, min(sy, n - ncen));
           const float* wt = a.centWeightDim == 2 ? s_cw
                             : (a.centWeightDim == 4 ? a.centWeight + (long long)i * mm : nullptr);
-          const float sgn = (wt == nullptr && a.cob != 1) ? -1.f : 1.f;
+          const float sgn = wt == nullptr ? -1.f : 1.f;
           float sum = 0.f;
           for (int r = sy; r < sy + ncen; r++)
             for (int c = sx; c < sx + ncen; c++) {

@@ -22,6 +22,7 @@
 #include "engine_internal.h"
 #include "gemm_form.h"
 #include "refnoise.h"
+#include "wfs_form.cuh"
 #include "wfs_launch.cuh"
 
 using namespace shwfs;
@@ -92,11 +93,14 @@ std::vector<T> to_host(const shwfs_array& a) {
 
 }  // namespace
 
-// a fused-kernel launch of one handle held back for a multi-handle launch
-struct DeferredPlain {
+// an FP32 formation launch of one handle held back for a multi-handle launch
+struct DeferredForm {
   struct shwfs_handle* h;
   shwfs::WfsArgs a;
-  long long ntiles;
+  const shwfs::FormEntry* entry;
+  int smem;           // at the multi-handle launch's shape
+  long long ngroups;  // groups of entry->maxS subaperture-frames
+  bool post;          // the noise/centroid kernel follows
 };
 
 struct shwfs_handle {
@@ -185,10 +189,10 @@ struct shwfs_handle {
   DevBuf<float> d_iscale;  // fp16 form: 1 / (sum of the subaperture's pupil)^2
   DevBuf<float> d_pupT;    // tensor-core forms: pupil by pixel group [ppr/8][nlit][8]
   cudaEvent_t splitEvent = nullptr;  // recorded between image formation and post stages
-  // while a multi-sensor batch captures: where the fused FP32 kernel's
+  // while a multi-sensor batch captures: where the FP32 formation kernel's
   // launch goes instead of the stream (the batch launches the kernels of
   // several handles of one instantiation as one multi-handle kernel)
-  std::vector<struct DeferredPlain>* plainSink = nullptr;
+  std::vector<struct DeferredForm>* formSink = nullptr;
   const PoisTab* poisTab = nullptr;  // Poisson CDF tables on this device
   // correlation centroiding: pattern (host copy), its size, the per-mode
   // device kernel, and the corrimg output (borrowed; device mirror)
@@ -841,6 +845,78 @@ shwfs_status enqueue_corr(shwfs_handle* h, float* cents, float* bimg, int nframe
   return SHWFS_OK;
 }
 
+// the warp form's instantiation for this handle's FP32 formation, or null
+// when it takes the block form (wfs_plain.cuh)
+const FormEntry* form_entry(const shwfs_handle* h) {
+  const int N = h->fftsize;
+  if (N % 2 || 2 * h->phasesize > N || h->phaseAmp || h->opticalBinning == 1 || h->nimg > h->clipsize) return nullptr;
+  int F = 1;
+  if (h->psfDim) {
+    if (h->psfsize != N || h->padded != N || h->preBin > 1 || h->clipsize != N) return nullptr;
+    if (2 * h->nimg == N) F = 2;
+  } else if (h->clipsize > N) {
+    return nullptr;
+  }
+  const auto& reg = form_registry();
+  const auto it = reg.find(FormKey{N, h->psfDim ? N : 0, F});
+  return it == reg.end() ? nullptr : &it->second;
+}
+
+int form_smem(const shwfs_handle* h, int S, int warps) {
+  return (form_const_floats(h->fftsize, h->psfDim ? h->psfsize : 0, h->phasesize, h->clipsize, h->nimg, h->psfDim == 2,
+                            h->centWeightDim == 2) +
+          warps * form_warp_floats(h->fftsize, S, h->nimg, h->ncen)) *
+         (int)sizeof(float);
+}
+
+// Launch shape of the warp form over nwork subaperture-frames.  A group's
+// time hardly depends on how many subapertures it holds (its transforms fill
+// idle lanes), so few subaperture-frames are spread one to a warp, and the
+// groups are filled once every SM has about eight warps' worth of them; as
+// many warps per CTA, up to four, as leave no SM without a CTA.
+struct FormShape {
+  int S, warps, smem, grid;
+};
+bool form_shape(const shwfs_handle* h, const FormEntry* e, long long nwork, FormShape* f) {
+  const long long perSM = (nwork + h->numSMs - 1) / h->numSMs;
+  f->S = (int)std::max<long long>(1, std::min<long long>(e->maxS, (perSM + 7) / 8));
+  const long long groups = (nwork + f->S - 1) / f->S;
+  f->warps = (int)std::max<long long>(1, std::min<long long>(kFormWarps, (groups + h->numSMs - 1) / h->numSMs));
+  while (f->warps > 1 && form_smem(h, f->S, f->warps) > 227 * 1024) f->warps--;
+  f->smem = form_smem(h, f->S, f->warps);
+  if (f->smem > 227 * 1024) return false;
+  int ctas = 0;
+  if (e->occupancy(&ctas, 32 * f->warps, f->smem) != cudaSuccess || ctas < 1) return false;
+  f->grid = (int)std::max<long long>(
+      1, std::min<long long>((groups + f->warps - 1) / f->warps, (long long)h->numSMs * ctas));
+  return true;
+}
+
+// the formation kernel over the frames of a (its mode says what it leaves)
+shwfs_status launch_form(const shwfs_handle* h, const FormEntry* e, WfsArgs a, cudaStream_t st) {
+  FormShape f;
+  if (!form_shape(h, e, (long long)a.nlit * a.nframes, &f))
+    return fail(SHWFS_ERR_UNSUPPORTED, "formation kernel cannot be resident");
+  a.TS = f.S;
+  CK(e->launch(a, f.grid, 32 * f.warps, f.smem, st));
+  return SHWFS_OK;
+}
+
+// whether the handle's formation runs the warp form
+const FormEntry* form_active(const shwfs_handle* h, long long nwork) {
+  const FormEntry* e = form_entry(h);
+  FormShape f;
+  return e && nwork > 0 && form_shape(h, e, nwork, &f) ? e : nullptr;
+}
+
+// whether the warp form finishes a frame itself: nothing is drawn and the
+// centroids, if any, are the window CoG; otherwise it leaves the pre-noise
+// images and the noise/centroid kernel follows
+bool form_finishes(const shwfs_handle* h, const WfsArgs& a) {
+  if (h->calsource == 0 && (h->addPoisson == 1 || h->readNoise != 0.f || h->useBrightest != 0 || h->ubIsArr)) return false;
+  return a.imageOnly || a.skipCents || (a.fitSize == 0 && a.gaussianFit <= 0 && a.cob == 0);
+}
+
 // queue one readout over nframes frames (device pointers)
 // device-side state a readout needs that is built lazily (the fit matrix);
 // run before a graph capture so that nothing allocates while capturing
@@ -889,7 +965,11 @@ shwfs_status enqueue_readout(shwfs_handle* h, const float* phs, float* cents, fl
     if (nframes != 1) return fail(SHWFS_ERR_UNSUPPORTED, "reference-stream noise runs one frame at a time");
     if (nlit) {
       WfsArgs a = make_args(h, phs, cents, bimg, 1, phsStride, kForm | kStorePreNoise);
-      CK(h->entry->launch(a, grid, h->smem, st));
+      if (const FormEntry* fe = form_active(h, nwork)) {
+        if (shwfs_status s = launch_form(h, fe, a, st)) return s;
+      } else {
+        CK(h->entry->launch(a, grid, h->smem, st));
+      }
     }
     RefNoiseArgs r{};
     r.nthreads = h->nthreads;
@@ -932,16 +1012,46 @@ shwfs_status enqueue_readout(shwfs_handle* h, const float* phs, float* cents, fl
       a.statusIn = h->d_status.p;
       a.statusOut = h->h_statusDev;
       CK(launch_post(a, h->numSMs, st, &postDone));
+    } else if (const FormEntry* fe = form_active(h, nwork)) {
+      WfsArgs a = make_args(h, phs, cents, bimg, nframes, phsStride, kForm | kPost);
+      const bool whole = form_finishes(h, a);
+      if (whole) {
+        // each final image is written once: straight to the host array when
+        // there is one
+        plainDirect = bimgHost != nullptr;
+        if (plainDirect) a.bimg = bimg = bimgHost;
+        if (!a.imageOnly) {
+          a.zeroUnlit = a.nunlit > 0;
+          postDone |= kPostDidUnlit;
+        }
+      } else {
+        a.mode = kForm | kStorePreNoise;
+        a.poisFlag = nullptr;
+      }
+      if (h->formSink && !bimgHost) {
+        h->formSink->push_back(DeferredForm{h, a, fe, form_smem(h, fe->maxS, kFormWarps),
+                                            (nwork + fe->maxS - 1) / fe->maxS, !whole});
+        if (!whole) postDone |= kPostDidUnlit;  // by the noise/centroid kernel behind the deferred launch
+      } else {
+        if (shwfs_status s = launch_form(h, fe, a, st)) return s;
+        if (!whole) {
+          a.mode = kNoiseCounter | kPost;
+          a.bimgOut = bimgHost;
+          CK(launch_post(a, h->numSMs, st, &postDone));
+          // the lit images are in the host array: the unlit kernel's
+          // (imageOnly) follow them there
+          if (bimgHost && (postDone & kPostDidOut)) {
+            plainDirect = true;
+            bimg = bimgHost;
+          }
+        }
+      }
     } else if (nlit) {
-      // the fused kernel writes each final image once: straight to the
-      // host array when there is one
+      // the block form writes each final image once too
       plainDirect = bimgHost != nullptr;
       if (plainDirect) bimg = bimgHost;
       WfsArgs a = make_args(h, phs, cents, bimg, nframes, phsStride, kForm | kNoiseCounter | kPost);
-      if (h->plainSink && !plainDirect)
-        h->plainSink->push_back(DeferredPlain{h, a, ntiles});
-      else
-        CK(h->entry->launch(a, grid, h->smem, st));
+      CK(h->entry->launch(a, grid, h->smem, st));
     }
     if (!h->unlit.empty() && !(postDone & kPostDidUnlit)) {
       WfsArgs a = make_args(h, phs, cents, bimg, nframes, phsStride, 0);
@@ -1015,7 +1125,11 @@ shwfs_status enqueue_physical(shwfs_handle* h, const float* phs, int state, cuda
       const int grid =
           (int)std::max<long long>(1, std::min<long long>(ntiles, (long long)h->numSMs * h->ctasPerSM));
       WfsArgs a = make_args(h, phs, h->d_cents.p, h->d_sub.p, 1, 0, kForm | kStorePreNoise);
-      CK(h->entry->launch(a, grid, h->smem, st));
+      if (const FormEntry* fe = form_active(h, nlit)) {
+        if (shwfs_status s = launch_form(h, fe, a, st)) return s;
+      } else {
+        CK(h->entry->launch(a, grid, h->smem, st));
+      }
     }
   }
   const bool first = state == 0 || state == -1, ro = state == 2 || state == -1;
@@ -1979,25 +2093,27 @@ shwfs_status batch_capture(shwfs_batch* b) {
   b->drop_graph();
   for (shwfs_handle* h : b->hs)
     if (shwfs_status s = prepare_readout(h)) return s;
-  // handles whose readout is one fused FP32 kernel plus independent work
-  // (counter noise, no correlation, no phase interpolation) and that share
-  // an instantiation with another such handle: their fused kernels run as
-  // one multi-handle launch on a branch of their own
-  std::vector<DeferredPlain> deferred;
+  // handles whose FP32 formation runs the warp form (counter noise, no
+  // correlation, no phase interpolation) and that share an instantiation and
+  // its shared-memory footprint (so that the multi-handle launch keeps each
+  // handle's occupancy) with another such handle: their formation kernels run
+  // as one multi-handle launch on a branch of their own
+  std::vector<DeferredForm> deferred;
+  auto multi_ok = [&](const shwfs_handle* h) -> const FormEntry* {
+    if (!b->multiEnabled || !h->entry || gemm_active(h) || h->noiseMode != SHWFS_NOISE_COUNTER || corr_active(h) ||
+        h->interp || h->lit.empty())
+      return nullptr;
+    const FormEntry* e = form_active(h, (long long)h->lit.size());
+    return e && form_smem(h, e->maxS, kFormWarps) <= 227 * 1024 ? e : nullptr;
+  };
   for (shwfs_handle* h : b->hs) {
-    h->plainSink = nullptr;
-    const bool ok = b->multiEnabled && h->entry && !gemm_active(h) && h->noiseMode == SHWFS_NOISE_COUNTER && !corr_active(h) &&
-                    !h->interp && !h->lit.empty();
-    if (!ok) continue;
-    // same instantiation and the same shared-memory footprint (so that the
-    // multi-handle launch keeps each handle's occupancy)
+    h->formSink = nullptr;
+    const FormEntry* e = multi_ok(h);
+    if (!e) continue;
     int same = 0;
     for (shwfs_handle* o : b->hs)
-      same += (o->entry == h->entry && o->smem == h->smem && !gemm_active(o) && o->noiseMode == SHWFS_NOISE_COUNTER &&
-               !corr_active(o) && !o->interp && !o->lit.empty())
-                  ? 1
-                  : 0;
-    if (same >= 2) h->plainSink = &deferred;
+      same += multi_ok(o) == e && form_smem(o, e->maxS, kFormWarps) == form_smem(h, e->maxS, kFormWarps) ? 1 : 0;
+    if (same >= 2) h->formSink = &deferred;
   }
   b->multiLaunches = 0;
   CK(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeRelaxed));
@@ -2016,37 +2132,45 @@ shwfs_status batch_capture(shwfs_batch* b) {
     }
     if (!deferred.empty()) {
       CK(cudaStreamWaitEvent(b->multiBranch, b->ev[0], 0));
-      // groups of one instantiation, at most kPlainMulti handles each
+      // groups of one instantiation, at most kFormMulti handles each
       std::vector<bool> done(deferred.size(), false);
       for (size_t i = 0; i < deferred.size(); i++) {
         if (done[i]) continue;
+        const FormEntry* e = deferred[i].entry;
         std::vector<size_t> grp;
-        for (size_t j = i; j < deferred.size() && grp.size() < (size_t)kPlainMulti; j++)
-          if (!done[j] && deferred[j].h->entry == deferred[i].h->entry && deferred[j].h->smem == deferred[i].h->smem)
-            grp.push_back(j);
-        int smem = 0, numSMs = deferred[i].h->numSMs;
-        for (size_t j : grp) {
-          done[j] = true;
-          smem = std::max(smem, deferred[j].h->smem);
-        }
+        for (size_t j = i; j < deferred.size() && grp.size() < (size_t)kFormMulti; j++)
+          if (!done[j] && deferred[j].entry == e && deferred[j].smem == deferred[i].smem) grp.push_back(j);
+        for (size_t j : grp) done[j] = true;
         int ctas = 0;
-        CK(deferred[i].h->entry->occupancy_multi(&ctas, smem));
+        CK(e->occupancy_multi(&ctas, 32 * kFormWarps, deferred[i].smem));
         if (ctas < 1) return fail(SHWFS_ERR_UNSUPPORTED, "multi-handle kernel cannot be resident");
         // each handle gets the CTAs a launch of its own would have (the
         // block scheduler then balances the union as it balances
         // concurrent launches)
-        const long long perHandle = (long long)numSMs * ctas;
-        PlainMulti m{};
+        const long long perHandle = (long long)deferred[i].h->numSMs * ctas;
+        FormMulti m{};
         m.n = (int)grp.size();
         m.ctaStart[0] = 0;
         for (size_t k = 0; k < grp.size(); k++) {
-          const long long t = deferred[grp[k]].ntiles;
+          const long long t = (deferred[grp[k]].ngroups + kFormWarps - 1) / kFormWarps;
           const long long c = std::max<long long>(1, std::min<long long>(t, perHandle));
           m.a[k] = deferred[grp[k]].a;
+          m.a[k].TS = e->maxS;
           m.ctaStart[k + 1] = m.ctaStart[k] + (int)c;
         }
-        CK(deferred[i].h->entry->launch_multi(m, smem, b->multiBranch));
+        CK(e->launch_multi(m, 32 * kFormWarps, deferred[i].smem, b->multiBranch));
         b->multiLaunches++;
+        for (size_t k : grp)
+          if (deferred[k].post) {
+            WfsArgs pa = deferred[k].a;
+            pa.mode = kNoiseCounter | kPost;
+            unsigned didPost = 0;
+            CK(launch_post(pa, deferred[k].h->numSMs, b->multiBranch, &didPost));
+            if (pa.nunlit > 0 && !(didPost & kPostDidUnlit)) {
+              pa.mode = 0;
+              CK(launch_unlit(pa, pa.unlit, pa.nunlit, b->multiBranch));
+            }
+          }
       }
       CK(cudaEventRecord(b->multiJoin, b->multiBranch));
       CK(cudaStreamWaitEvent(b->cap, b->multiJoin, 0));
@@ -2055,7 +2179,7 @@ shwfs_status batch_capture(shwfs_batch* b) {
     return SHWFS_OK;
   };
   const shwfs_status s = body();
-  for (shwfs_handle* h : b->hs) h->plainSink = nullptr;
+  for (shwfs_handle* h : b->hs) h->formSink = nullptr;
   const std::string err = g_err;
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(b->cap, &g);
@@ -2242,6 +2366,11 @@ shwfs_status shwfs_autotune(shwfs_handle* h, int* best_tile) {
   }
   if (h->lit.empty() || is_none(h->phs) || h->noiseMode == SHWFS_NOISE_REFERENCE) {
     // nothing to choose: no phase-input launches on this handle
+    if (best_tile) *best_tile = h->TS;
+    return SHWFS_OK;
+  }
+  if (form_active(h, (long long)h->lit.size())) {
+    // the warp form's launch shape follows from the number of subapertures
     if (best_tile) *best_tile = h->TS;
     return SHWFS_OK;
   }

@@ -1,4 +1,7 @@
-// Fused FP32 Shack-Hartmann WFS kernel ("plain" form).
+// Fused FP32 Shack-Hartmann WFS kernel, block form: the general one, for what
+// the warp form (wfs_form.cuh) does not cover -- odd FFT sizes, a spot PSF of
+// another size than the FFT, pre-binning, cropped convolutions,
+// phase+amplitude input, optical binning -- and for post-only launches.
 //
 // One CTA works on tiles of TS lit subapertures (several frames may share a
 // tile).  Everything between the phase read and the bimg/cents write stays in
@@ -441,11 +444,9 @@ __device__ __forceinline__ void post_tile(const WfsArgs& a, int ns, const int* s
     }
 }
 
-// The fused kernel's work for one handle, run by CTA `cta` of the `nctas`
-// CTAs that share its tiles (the whole grid for a single handle, a slice of
-// it in a multi-handle launch).
 template <int N, int P>
-__device__ __forceinline__ void plain_body(const WfsArgs& a, long long cta, long long nctas) {
+__global__ void __launch_bounds__(kThreads) wfs_plain_kernel(const __grid_constant__ WfsArgs a) {
+  const long long cta = blockIdx.x, nctas = gridDim.x;
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
   const int tid = threadIdx.x;
@@ -823,28 +824,6 @@ __device__ __forceinline__ void plain_body(const WfsArgs& a, long long cta, long
 #undef AMPSUM
 #undef SCAL
   }
-}
-
-template <int N, int P>
-__global__ void __launch_bounds__(kThreads) wfs_plain_kernel(const __grid_constant__ WfsArgs a) {
-  plain_body<N, P>(a, blockIdx.x, gridDim.x);
-}
-
-// Several handles of one (fftsize, psfsize) instantiation in one launch (the
-// multi-sensor batches): handle h owns CTAs [ctaStart[h], ctaStart[h+1]) and
-// each of them loops over that handle's tiles, as in a launch of its own.
-constexpr int kPlainMulti = 8;
-struct PlainMulti {
-  WfsArgs a[kPlainMulti];
-  int ctaStart[kPlainMulti + 1];
-  int n;
-};
-
-template <int N, int P>
-__global__ void __launch_bounds__(kThreads) wfs_plain_multi_kernel(const __grid_constant__ PlainMulti m) {
-  int h = 0;
-  while (h + 1 < m.n && (int)blockIdx.x >= m.ctaStart[h + 1]) h++;
-  plain_body<N, P>(m.a[h], (long long)blockIdx.x - m.ctaStart[h], (long long)(m.ctaStart[h + 1] - m.ctaStart[h]));
 }
 
 // launcher of the unlit-subaperture kernel (wfs_unlit.cu)

@@ -65,8 +65,9 @@ enum {
   /* extension (no reference counterpart): noise generator selection,
    * ival = SHWFS_NOISE_COUNTER or SHWFS_NOISE_REFERENCE */
   SHWFS_NOISEMODE = 100,
-  /* extension: subapertures per CTA tile of the fused kernel, ival = 0 picks
-   * the default for the geometry */
+  /* extension: subapertures per CTA tile of the FP32 form's block kernel (the
+   * geometries its warp kernel does not cover), ival = 0 picks the default for
+   * the geometry */
   SHWFS_TILESUBAPS = 101,
   /* extension: compute form, ival = SHWFS_FORM_* */
   SHWFS_FORM = 102,
@@ -213,9 +214,9 @@ typedef struct shwfs_value {
 typedef struct shwfs_info {
   int nsubx, nsubaps, nlit;
   int fftsize, psfsize, clipsize, nimg, phasesize;
-  int tile_subaps;      /* subapertures per CTA tile of the fused kernel */
-  int smem_bytes;       /* dynamic shared memory per CTA */
-  int grid_ctas;        /* CTAs launched per frame */
+  int tile_subaps;      /* subapertures per CTA tile of the FP32 block kernel */
+  int smem_bytes;       /* its dynamic shared memory per CTA */
+  int grid_ctas;        /* its CTAs per frame */
   int noise_mode;
   int cur_integ;
   uint64_t frames_read; /* readout frames processed (noise counter) */
@@ -326,11 +327,11 @@ const char* shwfs_version(void);
  * handle's persistent kernel(s) on its own graph branch, branches running
  * concurrently, so WFSs of different subaperture counts, FFT sizes and spot
  * PSFs go to the GPU with one graph launch.  With shwfs_batch_set_multi,
- * handles on the fused FP32 kernel that share its (fftsize, psfsize)
+ * handles whose FP32 image formation runs the warp form and that share its
  * instantiation and shared-memory footprint (counter noise, no correlation
- * centroiding, no phase interpolation) run as one persistent multi-handle
- * kernel over their tiles (up to 8 handles per launch) on a branch of its
- * own; results are identical either way.  Every handle must have
+ * centroiding, no phase interpolation) have their formation run as one
+ * persistent multi-handle kernel (up to 8 handles per launch) on a branch of
+ * its own; results are identical either way.  Every handle must have
  * device-resident phs/cents/bimg.
  * The graph is re-captured when a handle is updated; noise frame counters
  * advance on the device between replays. */
@@ -338,16 +339,17 @@ typedef struct shwfs_batch shwfs_batch;
 shwfs_status shwfs_batch_create(shwfs_handle* const* handles, int n, shwfs_batch** out);
 shwfs_status shwfs_batch_run(shwfs_batch* b, void* stream);
 shwfs_status shwfs_batch_free(shwfs_batch* b);
-/* on != 0: group handles into multi-handle fused-kernel launches (off by
+/* on != 0: group handles into multi-handle formation launches (off by
  * default: on the measured workloads the concurrent per-handle launches were
  * as fast or faster); re-captures the graph */
 shwfs_status shwfs_batch_set_multi(shwfs_batch* b, int on);
-/* multi-handle fused-kernel launches in the batch's captured graph */
+/* multi-handle formation launches in the batch's captured graph */
 shwfs_status shwfs_batch_multi_launches(const shwfs_batch* b, int* n);
 
 /* Time the handle's phase-input kernels over their launch shapes on scratch
- * buffers and keep the fastest: for the FP32 form the candidate tile sizes
- * of the fused kernel (*best_tile receives the one kept); for a tensor-core
+ * buffers and keep the fastest: for the FP32 form's block kernel the candidate
+ * tile sizes (*best_tile receives the one kept; the warp kernel's launch shape
+ * follows from the number of subapertures); for a tensor-core
  * form every staging of the GEMM kernel that fits (GEMM1 output-chunk width,
  * W2 chunk width, double buffering of the field and |F|^2 operands, Kc
  * stages, W2 ring depth; shwfs_info.gemm_* report the one kept).  Results are

@@ -165,6 +165,11 @@ __device__ __forceinline__ U4 philox4x32_10_rk(U4 c, const PhiloxKeys& K) {
 __device__ __forceinline__ float u32_to_uniform(uint32_t w) {
   return ((float)(w >> 8) + 0.5f) * (1.0f / 16777216.0f);
 }
+// the same value by one multiply-add (one rounding at either scale); in an
+// expression of its own, where the compiler cannot contract it differently
+__device__ __forceinline__ float u32_to_uniform_fma(uint32_t w) {
+  return fmaf((float)(w >> 8), 1.0f / 16777216.0f, 0.5f / 16777216.0f);
+}
 
 // Sequential uniform stream for one (frame, subap, pixel, purpose).
 struct CounterStream {
@@ -338,8 +343,10 @@ __device__ __forceinline__ int poisson_table_int(const PoisTab& T, int L, uint32
 
 // Poisson(d), 0 <= d < 1, by inversion of the uniform u4: the smallest j
 // with u4 <= F_j, F_j the CDF (d = 0 gives F_0 = 1, hence j = 0, without a
-// branch); the first four terms without branches
-__device__ __forceinline__ int poisson_frac(float d, float u4) {
+// branch).  poisson_frac_head: the first four terms without branches; *over
+// when u4 lies beyond them (probability < 2 %), and poisson_frac_tail then
+// gives the draw.
+__device__ __forceinline__ int poisson_frac_head(float d, float u4, bool* over) {
   float t = __expf(-d), F = t;
   int k2 = u4 > F ? 1 : 0;
   t *= d;
@@ -350,16 +357,29 @@ __device__ __forceinline__ int poisson_frac(float d, float u4) {
   k2 += u4 > F ? 1 : 0;
   t *= d * (1.0f / 3.0f);
   F += t;
-  if (u4 > F) {
-    int j = 3;
-    while (u4 > F && j < 40) {
-      j++;
-      t *= __fdividef(d, (float)j);
-      F += t;
-    }
-    k2 = j;
-  }
+  *over = u4 > F;
   return k2;
+}
+__device__ __forceinline__ int poisson_frac_tail(float d, float u4) {
+  float t = __expf(-d), F = t;
+  t *= d;
+  F += t;
+  t *= d * 0.5f;
+  F += t;
+  t *= d * (1.0f / 3.0f);
+  F += t;
+  int j = 3;
+  while (u4 > F && j < 40) {
+    j++;
+    t *= __fdividef(d, (float)j);
+    F += t;
+  }
+  return j;
+}
+__device__ __forceinline__ int poisson_frac(float d, float u4) {
+  bool over;
+  const int k = poisson_frac_head(d, u4, &over);
+  return over ? poisson_frac_tail(d, u4) : k;
 }
 
 __device__ __forceinline__ float poisson_tab(const PoisTab& T, uint32_t w3, float u4, float lam) {
@@ -445,7 +465,7 @@ __device__ __forceinline__ U4 quad_block(const PhiloxKeys& K, uint32_t frame, ui
 // two standard normal deviates from two words (Box-Muller: cosine and sine
 // branch of one pair)
 __device__ __forceinline__ void normal_pair(uint32_t w1, uint32_t w2, float& g0, float& g1) {
-  const float u1 = u32_to_uniform(w1), u2 = u32_to_uniform(w2);
+  const float u1 = u32_to_uniform_fma(w1), u2 = u32_to_uniform_fma(w2);
   const float q = -2.0f * __logf(u1);  // > 0: u1 < 1
   const float r = q * rsqrtf(q);
   float sn, cs;
@@ -490,10 +510,22 @@ __device__ __forceinline__ void quad_poisson(const PhiloxKeys& K, uint32_t frame
     lam[k] = ((skip >> k) & 1u) ? 0.0f : fmaxf(v[k], 0.0f);
     kt[k] = poisson_table_int(T, (int)lam[k], ws[k]);
   }
+  // (the tails of all four in one divergent region)
+  unsigned far = 0;
 #pragma unroll
-  for (int k = 0; k < 4; k++)
-    if (!((skip >> k) & 1u))
-      v[k] = (float)(kt[k] + poisson_frac(lam[k] - (float)(int)lam[k], u32_to_uniform(us[k])));
+  for (int k = 0; k < 4; k++) {
+    bool over;
+    const int j = poisson_frac_head(lam[k] - (float)(int)lam[k], u32_to_uniform_fma(us[k]), &over);
+    far |= over ? 1u << k : 0u;
+    const float x = (float)(kt[k] + j);
+    v[k] = ((skip >> k) & 1u) ? v[k] : x;
+  }
+  if (far) {
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if ((far >> k) & 1u)  // (a skipped pixel has lam 0 and is never here)
+        v[k] = (float)(kt[k] + poisson_frac_tail(lam[k] - (float)(int)lam[k], u32_to_uniform_fma(us[k])));
+  }
 }
 
 // shot noise of a pixel with lambda >= 64 from its own stream (PTRS)

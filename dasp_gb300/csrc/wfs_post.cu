@@ -205,18 +205,20 @@ __global__ void __launch_bounds__(kPostThreads, 3) wfs_post_kernel(const WfsArgs
   }
 }
 
-constexpr int kWarpThreads = 256;  // 8 warps per CTA
+// most warps per CTA (one CTA per SM when a batch fills it): 80 registers with
+// the Poisson sampler, 64 without
+constexpr int warp_max_warps(bool pois) { return pois ? 24 : 32; }
 constexpr int kWarpQ = 160;        // queued bright pixels per warp (at most 32 + one round's 128); even
 constexpr int kWarpMaxK = 16;      // subaperture-frames per chunk
 
-// Per-warp shared memory: two pixel buffers of bufPx floats (the chunk being
-// drawn and the next one, copied in asynchronously), the chunk's item table
-// for both buffers (per item an int4 {subaperture, noise frame index,
+// Per-warp shared memory in floats: the chunk's pixels (twice without Poisson
+// noise: the next chunk's are copied in meanwhile), the item tables of this
+// chunk and the next (per item an int4 {subaperture, noise frame index,
 // Poisson flag, frame} and the 64-bit offset of its image in bimg), the
 // window-row partial sums of the centroids and the bright-pixel queue
-// (kWarpQ 16-bit indices into the chunk's buffer).
-__host__ __device__ inline int warp_smem_floats(int bufPx, int ncen) {
-  return 2 * bufPx + 2 * 6 * kWarpMaxK + 2 * kWarpMaxK * ncen + kWarpQ / 2;
+// (kWarpQ 16-bit indices into the chunk's pixels, and their number).
+__host__ __device__ inline int warp_smem_floats(bool pois, int K, int mm, int ncen) {
+  return (pois ? 1 : 2) * ((K * mm + 3) & ~3) + 2 * 6 * K + ((2 * K * ncen + 3) & ~3) + kWarpQ / 2 + 4;
 }
 
 // The common configuration (window CoG or image only; no brightest-pixel
@@ -224,36 +226,44 @@ __host__ __device__ inline int warp_smem_floats(int bufPx, int ncen) {
 // lit subaperture-frames: the chunk's pixels are drawn a quad (four
 // consecutive pixels of one image) per lane, lanes over the chunk's
 // flattened quad index (every lane busy whatever nimg is), with 16-byte
-// loads and stores when nimg^2 is a multiple of 4.  Bright pixels
-// (lambda >= 64, the rejection sampler) are queued and drawn by the whole
-// warp after a round that left more than 32 in the queue and after the
+// loads (a round ahead; without Poisson noise the chunk ahead, by cp.async:
+// the rounds are then too short to hide a load) and stores when nimg^2 is a
+// multiple of 4.  Bright
+// pixels (lambda >= 64, the rejection sampler) are queued and drawn by the
+// whole warp after a round that left more than 32 in the queue and after the
 // last, then the window centroids come from the chunk's images in shared
-// memory.  Warps are independent (no block barrier after the table load);
-// each copies its next chunk into shared memory with cp.async while it
-// draws the current one.  Unlit subapertures are not visited; their
-// centroids are zeroed at the end (zeroUnlit).  Pixels and streams are
-// those of wfs_post_kernel and of the fused FP32 kernel (quad_normals,
-// quad_poisson, ptrs_pixel), so equal pre-noise images give equal noisy
-// images in every form.  RN (read noise on) and POIS (Poisson on) are
-// compile-time.
+// memory.  Warps are independent (no block barrier after the table load).
+// Unlit subapertures are not visited; their centroids are zeroed at the
+// end (zeroUnlit).  Pixels and streams are those of wfs_post_kernel and of
+// the fused FP32 kernel (quad_normals, quad_poisson, ptrs_pixel), so equal
+// pre-noise images give equal noisy images in every form.  RN (read noise on)
+// and POIS (Poisson on) are compile-time.
+//
+// Issue-bound on the samplers (205 MB of images in and out for 64 frames of
+// the 74x74 sensor: 31 us of memory time).  One CTA of 24 warps per SM holds
+// one copy of the Poisson table, which leaves a warp room for chunks of up to
+// 16 items: the rejection sampler then runs with several bright pixels per
+// drain (with three 8-warp CTAs and chunks of five items its drains, a fifth
+// of their lanes busy, took 75 of 267 us; now 23 of 179).  Without noise the
+// same launch takes 66 us.
 template <bool RN, bool POIS>
-__global__ void __launch_bounds__(kWarpThreads, 3)
-    wfs_post_warp_kernel(const WfsArgs a, const PoisTab* __restrict__ tab, int K, int bufPx) {
+__global__ void __launch_bounds__(32 * warp_max_warps(POIS), 1)
+    wfs_post_warp_kernel(const __grid_constant__ WfsArgs a, const PoisTab* __restrict__ tab, int K) {
   extern __shared__ __align__(16) float smem_post[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m = a.m, mm = m * m, ncen = a.ncen;
   const bool cw2d = a.centWeightDim == 2;
   PoisTab* s_tab = reinterpret_cast<PoisTab*>(smem_post);
   float* s_cw = smem_post + (POIS ? sizeof(PoisTab) / sizeof(float) : 0);
-  float* wbase = s_cw + ((cw2d ? mm : 0) + 3) / 4 * 4 + warp * warp_smem_floats(bufPx, ncen);
-  // buffer b: pixels wbase + b * bufPx, items item0 + b * kWarpMaxK, image
-  // offsets off0 + b * kWarpMaxK
-  int4* item0 = reinterpret_cast<int4*>(wbase + 2 * bufPx);
-  long long* off0 = reinterpret_cast<long long*>(item0 + 2 * kWarpMaxK);
-  float* s_rows = wbase + 2 * bufPx + 12 * kWarpMaxK;
-  // queued pixels as 16-bit indices into the chunk's buffer (bufPx <= 3200:
-  // the launcher's 200 KB bound on 16 buffers of bufPx floats)
-  unsigned short* q_idx = reinterpret_cast<unsigned short*>(s_rows + 2 * kWarpMaxK * ncen);
+  float* img0 = s_cw + ((cw2d ? mm : 0) + 3) / 4 * 4 + warp * warp_smem_floats(POIS, K, mm, ncen);
+  const int bufPx = (K * mm + 3) & ~3;  // pixel buffer b: img0 + b * bufPx (one with Poisson noise)
+  // table buffer b: items item0 + b * K, image offsets off0 + b * K
+  int4* item0 = reinterpret_cast<int4*>(img0 + (POIS ? 1 : 2) * bufPx);
+  long long* off0 = reinterpret_cast<long long*>(item0 + 2 * K);
+  float* s_rows = reinterpret_cast<float*>(off0 + 2 * K);
+  unsigned short* q_idx = reinterpret_cast<unsigned short*>(s_rows + ((2 * K * ncen + 3) & ~3));
+  int* q_n = reinterpret_cast<int*>(q_idx + kWarpQ);  // bright pixels queued
+  if (lane == 0) *q_n = 0;
   if constexpr (POIS) {
     const int4* src = reinterpret_cast<const int4*>(tab);
     int4* dst = reinterpret_cast<int4*>(s_tab);
@@ -261,12 +271,6 @@ __global__ void __launch_bounds__(kWarpThreads, 3)
   }
   if (cw2d)
     for (int k = tid; k < mm; k += blockDim.x) s_cw[k] = a.centWeight[k];
-  __syncthreads();
-  // launched programmatically behind the image-formation kernel: everything
-  // above reads constants only; bimg is read after that grid has completed
-  // and its writes are visible (a no-op for an ordinary launch)
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (a.statusOut && blockIdx.x == 0 && tid == 0) *(volatile int*)a.statusOut = *(const volatile int*)a.statusIn;
 
   const long long items = (long long)a.nlit * a.nframes;
   const long long nchunks = (items + K - 1) / K;
@@ -274,7 +278,6 @@ __global__ void __launch_bounds__(kWarpThreads, 3)
   const bool noise = a.mode & kNoiseCounter;
   const float rn = a.readNoise;
   const unsigned long long fbase = frame_base(a);
-  const bool vec = (mm & 3) == 0 && (a.bimgFrameStride & 3) == 0 && ((uintptr_t)a.bimg & 15) == 0;
   const bool cents = a.imageOnly == 0 && !a.skipCents;
   const int sx0 = (m - ncen) / 2;
   const float inv_mm = 1.0f / (float)mm, inv_nc = 1.0f / (float)ncen;
@@ -288,76 +291,95 @@ __global__ void __launch_bounds__(kWarpThreads, 3)
   // whole quads with 16-byte loads and stores
   const bool vec4 = (mm & 3) == 0 && (a.bimgFrameStride & 3) == 0 && ((uintptr_t)a.bimg & 15) == 0 &&
                     (!out2 || ((uintptr_t)a.bimgOut & 15) == 0);
+  const int nqi = (mm + 3) >> 2;  // quads per item
 
-  // item table of chunk c into buffer b's table (lanes < K), then its
-  // pixels into buffer b with cp.async (one commit group per lane, empty
-  // past the end)
-  // the first item of this warp's current chunk as (frame cf, lit index
-  // cl), advanced by whole strides of nw chunks without a division
+  // the first item of this warp's chunk as (frame cf, lit index cl), advanced
+  // by whole strides of nw chunks without a division
   long long cf = (gw * K) / a.nlit;
   int cl = (int)(gw * K - cf * a.nlit);
   const long long strideItems = nw * (long long)K;
   const long long sf = strideItems / a.nlit;
   const int sl = (int)(strideItems - sf * a.nlit);
-  auto issue = [&](long long c, int b, long long f0, int l0) {
-    int4* itb = item0 + b * kWarpMaxK;
-    long long* ofb = off0 + b * kWarpMaxK;
-    if (c < nchunks) {
-      const long long w0 = c * K;
-      const int nk = (int)min((long long)K, items - w0);
-      if (lane < nk) {
-        int li = l0 + lane, f = (int)f0;
-        while (li >= a.nlit) {
-          li -= a.nlit;
-          f++;
-        }
-        const int i = a.lit[li];
-        const int pf = POIS ? (a.totsig[i] > 0.f || a.sky * a.frac[i] > 0.f || a.skyArr != nullptr) : 0;
-        itb[lane] = make_int4(i, (int)(uint32_t)(fbase + (unsigned long long)f), pf, f);
-        ofb[lane] = (long long)f * a.bimgFrameStride + (long long)i * mm;
+  // chunk c's item table into buffer b
+  auto table = [&](long long c, int b) {
+    if (c < nchunks && lane < (int)min((long long)K, items - c * K)) {
+      int li = cl + lane, f = (int)cf;
+      while (li >= a.nlit) {
+        li -= a.nlit;
+        f++;
       }
-      __syncwarp();
-      float* dst = wbase + b * bufPx;
-      if (vec) {
-        const int nq = nk * mm / 4, q4 = mm / 4;
-        const float inv_q4 = 1.0f / (float)q4;
-        for (int q = lane; q < nq; q += 32) {
-          const int s = div_small(q, q4, inv_q4), r = q - s * q4;
-          const float* src = a.bimg + ofb[s] + 4 * r;
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + 4 * q)),
-                       "l"(src)
+      const int i = a.lit[li];
+      const int pf = POIS ? (a.totsig[i] > 0.f || a.sky * a.frac[i] > 0.f || a.skyArr != nullptr) : 0;
+      item0[b * K + lane] = make_int4(i, (int)(uint32_t)(fbase + (unsigned long long)f), pf, f);
+      off0[b * K + lane] = (long long)f * a.bimgFrameStride + (long long)i * mm;
+    }
+    __syncwarp();
+  };
+
+  // chunk c's pixels into buffer b (whole quads: 16 bytes at a time), one
+  // commit group per lane, empty past the end
+  auto prefetch = [&](long long c, int b) {
+    if (c < nchunks) {
+      const int nk = (int)min((long long)K, items - c * K);
+      const long long* offs = off0 + b * K;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(img0 + b * bufPx);
+      const int per = vec4 ? nqi : mm;  // copies per item
+      int s = 0, e = lane;
+      while (e >= per) {
+        e -= per;
+        s++;
+      }
+      for (int k = lane; k < nk * per; k += 32) {
+        if (vec4)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)k),
+                       "l"(a.bimg + offs[s] + 4 * e)
                        : "memory");
-        }
-      } else {
-        for (int g = lane; g < nk * mm; g += 32) {
-          const int s = div_small(g, mm, inv_mm), pix = g - s * mm;
-          const float* src = a.bimg + ofb[s] + pix;
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + g)),
-                       "l"(src)
+        else
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * (uint32_t)k),
+                       "l"(a.bimg + offs[s] + e)
                        : "memory");
+        e += 32;
+        while (e >= per) {
+          e -= per;
+          s++;
         }
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  int b = 0;
-  issue(gw, 0, cf, cl);
-  for (long long c = gw; c < nchunks; c += nw, b ^= 1) {
-    const long long w0 = c * K;
-    const int nk = (int)min((long long)K, items - w0);
-    cf += sf;  // the next chunk of this warp
+  table(gw, 0);
+  __syncthreads();
+  // launched programmatically behind the image-formation kernel: everything
+  // above reads constants only; bimg is read after that grid has completed
+  // and its writes are visible (a no-op for an ordinary launch)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (a.statusOut && blockIdx.x == 0 && tid == 0) *(volatile int*)a.statusOut = *(const volatile int*)a.statusIn;
+
+  auto advance = [&]() {  // (cf, cl) to the warp's next chunk
+    cf += sf;
     cl += sl;
     if (cl >= a.nlit) {
       cl -= a.nlit;
       cf++;
     }
-    issue(c + nw, b ^ 1, cf, cl);  // the next chunk's copies, in flight while this one is drawn
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncwarp();
-    float* img = wbase + b * bufPx;
-    const int4* items = item0 + b * kWarpMaxK;
-    const long long* offs = off0 + b * kWarpMaxK;
+  };
+  int b = 0;
+  if constexpr (!POIS) prefetch(gw, 0);
+  for (long long c = gw; c < nchunks; c += nw, b ^= 1) {
+    const int nk = (int)min((long long)K, items - c * K);
+    float* img = img0;
+    if constexpr (!POIS) {
+      // the next chunk's table and copies, in flight while this one is drawn
+      advance();
+      table(c + nw, b ^ 1);
+      prefetch(c + nw, b ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncwarp();
+      img += b * bufPx;
+    }
+    const int4* items_ = item0 + b * K;
+    const long long* offs = off0 + b * K;
     // noise, threshold, power and stores of one pixel (x: its mean; g: its
     // read-noise normal)
     auto finish = [&](float x, float g) {
@@ -369,52 +391,68 @@ __global__ void __launch_bounds__(kWarpThreads, 3)
       if (!pw1) x = a.pxlPower == 2.f ? x * x : powf(x, a.pxlPower);
       return x;
     };
-    int nq = 0;  // bright pixels queued (warp-uniform)
-    const int nqi = (mm + 3) >> 2, nqc = nk * nqi;  // quads per item, per chunk
+    const int nqc = nk * nqi;  // quads of the chunk
     // this lane's quad Q = Q0 + lane of the chunk is quad q of item s
     int s = 0, q = lane;
     while (q >= nqi) {
       q -= nqi;
       s++;
     }
-    // one round of 32 quads (the last may be partial)
-    auto round = [&](int Q0) {
-      const bool in = Q0 + lane < nqc;
-      const int si = in ? s : 0;
-      const int4 it = items[si];
-      (void)it;  // unused without noise
-      const int p0 = 4 * q, np = in ? min(4, mm - p0) : 0;
-      float* src = img + si * mm + p0;
-      float v[4];
-      if (vec4 && in) {
+    // the four pre-noise pixels of quad qq of item ss (0 past the image's end)
+    auto load = [&](int ss, int qq, float (&v)[4]) {
+      v[0] = v[1] = v[2] = v[3] = 0.f;
+      if (ss >= nk) return;
+      const float* src = POIS ? a.bimg + offs[ss] + 4 * qq : img + ss * mm + 4 * qq;
+      if (vec4) {
         const float4 t = *reinterpret_cast<const float4*>(src);
         v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
       } else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) v[k] = k < np ? src[k] : 0.f;
+        for (int k = 0; k < 4; k++)
+          if (4 * qq + k < mm) v[k] = src[k];
       }
-      unsigned bmask = 0;  // pixels with lambda >= 64, queued
+    };
+    float ahead[4];
+    if constexpr (POIS) load(s, q, ahead);
+    // one round of 32 quads (the last may be partial)
+    auto round = [&]() {
+      const int si = s, qi = q;
+      const bool in = si < nk;
+      float v[4];
       if constexpr (POIS) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const bool br = noise && k < np && it.z && v[k] >= kModalMaxLam;
-          const unsigned bm = __ballot_sync(0xffffffffu, br);
-          if (bm) {
-            if (br) {
-              bmask |= 1u << k;
-              const int slot = nq + __popc(bm & ((1u << lane) - 1u));
-              q_idx[slot] = (unsigned short)(si * mm + p0 + k);
-            }
-            nq += __popc(bm);
-          }
+        for (int k = 0; k < 4; k++) v[k] = ahead[k];
+      } else {
+        load(si, qi, v);
+      }
+      q += 32;
+      while (q >= nqi) {
+        q -= nqi;
+        s++;
+      }
+      if constexpr (POIS) load(s, q, ahead);  // the next round's
+      const int4 it = items_[in ? si : 0];
+      (void)it;  // unused without noise
+      const int p0 = 4 * qi, np = in ? min(4, mm - p0) : 0;
+      unsigned bmask = 0;  // pixels with lambda >= 64, queued
+      if constexpr (POIS) {
+        if (noise && it.z) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) bmask |= (k < np && v[k] >= kModalMaxLam) ? 1u << k : 0u;
+        }
+        // the queue's order does not matter: each pixel has its own stream
+        if (bmask) {
+          int slot = atomicAdd(q_n, __popc(bmask));
+          const int g0 = si * mm + p0;
+          for (unsigned rest = bmask; rest; rest &= rest - 1u) q_idx[slot++] = (unsigned short)(g0 + __ffs(rest) - 1);
         }
       }
       if (noise && in) {
         float g[4] = {0.f, 0.f, 0.f, 0.f};
-        if constexpr (RN) quad_normals(a.philoxKeys, (uint32_t)it.y, (uint32_t)it.x, (uint32_t)q, g);
+        if constexpr (RN) quad_normals(a.philoxKeys, (uint32_t)it.y, (uint32_t)it.x, (uint32_t)qi, g);
         if constexpr (POIS) {
           if (it.z) {
-            quad_poisson(a.philoxKeys, (uint32_t)it.y, (uint32_t)it.x, (uint32_t)q, *s_tab, v, bmask);
+            quad_poisson(a.philoxKeys, (uint32_t)it.y, (uint32_t)it.x, (uint32_t)qi, *s_tab, v, bmask);
           }
         }
         // a queued pixel keeps its mean (in img too) until the drain
@@ -429,54 +467,55 @@ __global__ void __launch_bounds__(kWarpThreads, 3)
       }
       if (in) {
         const long long ob = offs[si] + p0;
+        float* dst = img + si * mm + p0;
         // (queued pixels too: the drain overwrites them after a __syncwarp)
         if (vec4) {
           const float4 t = make_float4(v[0], v[1], v[2], v[3]);
           *reinterpret_cast<float4*>(a.bimg + ob) = t;
           if (out2) *reinterpret_cast<float4*>(a.bimgOut + ob) = t;
-          if (cents) *reinterpret_cast<float4*>(src) = t;
+          *reinterpret_cast<float4*>(dst) = t;
         } else {
 #pragma unroll
           for (int k = 0; k < 4; k++) {
             if (k < np) {
               a.bimg[ob + k] = v[k];
               if (out2) a.bimgOut[ob + k] = v[k];
-              if (cents) src[k] = v[k];
+              dst[k] = v[k];
             }
           }
         }
-      }
-      q += 32;
-      while (q >= nqi) {
-        q -= nqi;
-        s++;
       }
     };
     // the queued bright pixels, drawn by the whole warp: after a round that
     // left more than 32 (a round queues at most 128) and after the last round
     auto drain = [&]() {
       __syncwarp();
+      const int nq = *q_n;
       for (int k = lane; k < nq; k += 32) {
         const int g = q_idx[k];
         const int sq = div_small(g, mm, inv_mm), pq = g - sq * mm;
-        const int4 it = items[sq];
+        const int4 it = items_[sq];
         float gn = 0.f;
         if constexpr (RN) gn = pixel_normal(a.philoxKeys, (uint32_t)it.y, (uint32_t)it.x, (uint32_t)pq);
         const float x = finish(ptrs_pixel(a.philoxKeys, (uint32_t)it.y, (uint32_t)it.x, (uint32_t)pq, img[g]), gn);
         a.bimg[offs[sq] + pq] = x;
         if (out2) a.bimgOut[offs[sq] + pq] = x;
-        if (cents) img[g] = x;
+        img[g] = x;
       }
-      nq = 0;
+      __syncwarp();
+      if (lane == 0) *q_n = 0;
       __syncwarp();
     };
     // one copy of each in the loop: the samplers' code is large, and a
     // second copy of either (a separate last round, a drain after the loop)
     // overflowed the instruction cache
     for (int Q0 = 0; Q0 < nqc; Q0 += 32) {
-      round(Q0);
-      if constexpr (POIS)
+      round();
+      if constexpr (POIS) {
+        __syncwarp();
+        const int nq = *(volatile int*)q_n;
         if (nq > kWarpQ - 128 || (nq && Q0 + 32 >= nqc)) drain();
+      }
     }
     if (cents) {
       __syncwarp();
@@ -487,19 +526,20 @@ __global__ void __launch_bounds__(kWarpThreads, 3)
         const int r = sx0 + rr;
         const float* row = img + s * mm + r * m + sx0;
         const float* wrow = cw2d ? s_cw + r * m + sx0
-                                 : (a.centWeightDim == 4 ? a.centWeight + (long long)items[s].x * mm + r * m + sx0 : nullptr);
-        float ps = 0.f, px = 0.f;
+                                 : (a.centWeightDim == 4 ? a.centWeight + (long long)items_[s].x * mm + r * m + sx0 : nullptr);
+        float ps = 0.f, px = 0.f, x = (float)sx0;
         if (wrow) {
-          for (int c2 = 0; c2 < ncen; c2++) {
+          for (int c2 = 0; c2 < ncen; c2++, x += 1.f) {
             const float v = row[c2] * wrow[c2];
             ps += v;
-            px += v * (float)(sx0 + c2);
+            px += v * x;
           }
         } else {
-          for (int c2 = 0; c2 < ncen; c2++) {
+#pragma unroll 5
+          for (int c2 = 0; c2 < ncen; c2++, x += 1.f) {
             const float v = row[c2];
             ps += v;
-            px += v * (float)(sx0 + c2);
+            px += v * x;
           }
         }
         s_rows[2 * t] = ps;
@@ -507,22 +547,26 @@ __global__ void __launch_bounds__(kWarpThreads, 3)
       }
       __syncwarp();
       if (lane < nk) {
-        float sum = 0.f, sxv = 0.f, syv = 0.f;
-        for (int rr = 0; rr < ncen; rr++) {
+        float sum = 0.f, sxv = 0.f, syv = 0.f, y = (float)sx0;
+        for (int rr = 0; rr < ncen; rr++, y += 1.f) {
           const float ps = s_rows[2 * (lane * ncen + rr)];
           sum += ps;
           sxv += s_rows[2 * (lane * ncen + rr) + 1];
-          syv += ps * (float)(sx0 + rr);
+          syv += ps * y;
         }
         float cx = 0.f, cy = 0.f;
         if (sum > 0.f) {
           cx = sxv / sum - 0.5f * (float)(m - 1);
           cy = syv / sum - 0.5f * (float)(m - 1);
         }
-        calibrate_and_store(a, items[lane].x, items[lane].w, cx, cy);
+        calibrate_and_store(a, items_[lane].x, items_[lane].w, cx, cy);
       }
     }
-    __syncwarp();  // every lane is done with buffer b before it is refilled
+    if constexpr (POIS) {
+      advance();
+      table(c + nw, b ^ 1);
+    }
+    __syncwarp();  // every lane is done with the chunk's pixels and table
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   if (a.zeroUnlit) {
@@ -557,28 +601,38 @@ cudaError_t launch_post(const WfsArgs& a0, int numSMs, cudaStream_t stream, unsi
                       a.fitSize == 0 && a.gaussianFit <= 0 && a.cob == 0;
   const int tabB = pois ? (int)sizeof(PoisTab) : 0;
   const int cwB = ((a.centWeightDim == 2 ? mm : 0) + 3) / 4 * 16;
-  const int bufPx = (std::max(512, mm) + 3) / 4 * 4;
-  const int warpB = warp_smem_floats(bufPx, a.ncen) * (int)sizeof(float);
-  const int wsmem = tabB + cwB + (kWarpThreads / 32) * warpB;
-  if (simple && a.ncen >= 1 && wsmem <= 200 * 1024) {
+  // the warp kernel's launch shape: as many warps per SM as hold a
+  // chunk of one item, then the largest chunk that fits beside them
+  const int budget = (227 * 1024 - 1024) - tabB - cwB;
+  auto warpB = [&](int K) { return warp_smem_floats(pois, K, mm, std::max(1, a.ncen)) * (int)sizeof(float); };
+  const int maxWarps = std::min(warp_max_warps(pois), budget / warpB(1));
+  if (simple && a.ncen >= 1 && maxWarps >= 8) {
     const bool rnOn = a.calsource == 0 && a.readNoise != 0.f;
     auto kern = pois ? (rnOn ? wfs_post_warp_kernel<true, true> : wfs_post_warp_kernel<false, true>)
                      : (rnOn ? wfs_post_warp_kernel<true, false> : wfs_post_warp_kernel<false, false>);
     if (a.calsource != 0) a.readNoise = 0.f;
-    int ctas = 0;
-    cudaError_t e = kernel_smem_setup((const void*)kern, wsmem, kWarpThreads, &ctas);
-    if (e != cudaSuccess) return e;
-    if (ctas < 1) return cudaErrorInvalidConfiguration;
-    const long long cap = (long long)numSMs * ctas;
-    const long long warps = cap * (kWarpThreads / 32);
-    // chunk size: as many items as fill the buffer, fewer when that would
-    // leave resident warps without a chunk (small batches: latency)
-    int K = std::max(1, std::min(kWarpMaxK, bufPx / mm));
-    const long long perWarp = (nwork + warps - 1) / warps;
-    if (perWarp < K) K = (int)std::max(1LL, perWarp);
+    const long long all = (long long)numSMs * maxWarps;  // resident warps
+    // chunk size: of those that fit, the one that takes the resident warps the
+    // fewest rounds, counting a chunk's table and centroids as two more (a
+    // larger chunk fills its last round and the bright-pixel drains better, a
+    // smaller one the last sweep over the warps)
+    int K = 1;
+    long long best = 0;
+    for (int k = kWarpMaxK; k >= 1; k--) {
+      if (k > 1 && (maxWarps * warpB(k) > budget || k > (nwork + all - 1) / all)) continue;
+      const long long sweeps = ((nwork + k - 1) / k + all - 1) / all;
+      const long long cost = sweeps * ((k * ((mm + 3) / 4) + 31) / 32 + 2);
+      if (best == 0 || cost < best) {
+        best = cost;
+        K = k;
+      }
+    }
     const long long nchunks = (nwork + K - 1) / K;
-    const long long needCtas = (nchunks + kWarpThreads / 32 - 1) / (kWarpThreads / 32);
-    const int grid = (int)std::max(1LL, std::min(cap, needCtas));
+    const int warps = (int)std::max<long long>(1, std::min<long long>(maxWarps, (nchunks + numSMs - 1) / numSMs));
+    const int wsmem = tabB + cwB + warps * warpB(K);
+    const int grid = (int)std::max<long long>(1, std::min<long long>(numSMs, (nchunks + warps - 1) / warps));
+    cudaError_t e = kernel_smem_setup((const void*)kern, wsmem, 32 * warps, nullptr);
+    if (e != cudaSuccess) return e;
     if (done) {
       if (!a.imageOnly && a.unlit && a.nunlit > 0) {
         a.zeroUnlit = 1;
@@ -595,7 +649,7 @@ cudaError_t launch_post(const WfsArgs& a0, int numSMs, cudaStream_t stream, unsi
     // in griddepcontrol.wait after loading their tables
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kWarpThreads);
+    cfg.blockDim = dim3((unsigned)(32 * warps));
     cfg.dynamicSmemBytes = (size_t)wsmem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -604,7 +658,7 @@ cudaError_t launch_post(const WfsArgs& a0, int numSMs, cudaStream_t stream, unsi
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const PoisTab* tabArg = pois ? tab : nullptr;
-    return cudaLaunchKernelEx(&cfg, kern, a, tabArg, K, bufPx);
+    return cudaLaunchKernelEx(&cfg, kern, a, tabArg, K);
   }
   const int smem = (a.TS * mm + (a.centWeightDim == 2 ? mm : 0)) * (int)sizeof(float) +
                    (pois ? (int)sizeof(PoisTab) : 0);

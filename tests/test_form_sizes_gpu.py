@@ -44,7 +44,7 @@ def test_every_size(N, psf, images):
     # of a width that bins fractionally
     m = {"half": N // 2, "full": N, "ragged": N // 2 - 1}[images]
     c = Case(nsubx=5, p=N // 2, N=N, C=N, m=m, ncen=m, psf=psf, sig=1e4, skybrightness=2.0, noiseFloor=1.0,
-             phase_seed=N)
+             phase_seed=N, L0=2.0)
     _check(c)
 
 
@@ -54,7 +54,7 @@ def test_groups_and_grids(nsubx, frames, psf):
     # one subaperture per warp up to several, partial last groups, groups that
     # span frames, more groups than resident warps
     c = Case(nsubx=nsubx, p=8 if nsubx > 3 else 10, N=16 if nsubx > 3 else 20, psf=psf, sig=1e3, skybrightness=3.0,
-             noiseFloor=2.0, obs=0.1, phase_seed=nsubx)
+             noiseFloor=2.0, obs=0.1, phase_seed=nsubx, L0=2.0)
     _check(c, frames)
 
 

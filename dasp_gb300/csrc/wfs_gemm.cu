@@ -50,6 +50,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 #include <vector>
@@ -70,6 +71,8 @@ constexpr int kTileSubaps = 128;
 constexpr uint32_t kTmemCols = 512;
 constexpr long long kWaitCycles = 4000000000LL;  // about 2 s at the maximum SM clock
 constexpr uint32_t kLBO = 128;  // bytes between core matrices along K
+// dynamic limit: 227 KB minus the kernel's static shared memory (< 4 KB)
+constexpr uint32_t kGemmSmemLimit = 227 * 1024 - 4096;
 
 // TMEM columns: D1 buffers 0 and 1 at 0 and 128, D2 at 256 (N2 <= 256
 // columns), a third D1 buffer at 384 when N2 <= 128
@@ -150,7 +153,8 @@ struct Bars {
   uint64_t ehelp;  // the epilogue warps' share of the first tile's field
 };
 
-template <int FMT, int PASSES>
+// SMALL: tiles of g.TR live rows instead of 128 (small_launch)
+template <int FMT, int PASSES, bool SMALL>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     wfs_gemm_kernel(const WfsArgs a, const GemmGeom g, const float* __restrict__ iscale, int* err) {
   constexpr bool SPLIT = PASSES == 3;
@@ -225,7 +229,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   };
 
   const long long nwork = (long long)a.nlit * a.nframes;
-  const long long ntiles = (nwork + kTileSubaps - 1) / kTileSubaps;
+  const int TR = SMALL ? g.TR : kTileSubaps;
+  const long long ntiles = (nwork + TR - 1) / TR;
   const int myTiles = blockIdx.x < ntiles ? (int)((ntiles - 1 - blockIdx.x) / gridDim.x + 1) : 0;
   // the epilogue warps build half of the first tile's field, which their
   // first D1 chunk waits for anyway (the field warps go on to the next tile)
@@ -387,9 +392,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   } else {
     // ================= consumers =================
     // warps 0-7: epilogue (TMEM lane quarter warp & 3, column half h);
-    // warps 8-15: field build (row r, pixel-group parity h)
+    // warps 8-15: field build (row rf, every parts-th pixel group from part)
     const int r = tid & 127, h = (tid >> 7) & 1;
+    const int rf = tid & (TR - 1), parts = 256 / TR, part = (tid & 255) / TR;
     const bool fieldRole = warp >= kEpiWarps;
+    // rows from TR on are not built, read or stored: whatever the operand
+    // buffers hold there stays in their own accumulator rows
+    const bool liveLanes = !SMALL || 32 * (warp & 3) < TR;
     const bool vecPup = (pp & 3) == 0 && ((uintptr_t)a.pup & 15) == 0;
     const bool vecPhs = (p & 1) == 0 && (a.W & 1) == 0 && (a.phsFrameStride & 1) == 0 && ((uintptr_t)a.phs & 7) == 0;
     const bool vecOut = (mm & 3) == 0 && (a.bimgFrameStride & 3) == 0 && ((uintptr_t)a.bimg & 15) == 0;
@@ -399,11 +408,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       bool live;
       int sub, frm, li;
     };
-    // this thread's row (subaperture-frame) of tile lt
-    auto row_of = [&](int lt) {
+    // row (subaperture-frame) rr of tile lt
+    auto row_of = [&](int lt, int rr) {
       Row o{false, 0, 0, 0};
-      const long long w = (blockIdx.x + (long long)lt * gridDim.x) * kTileSubaps + r;
-      if (lt < myTiles && w < nwork) {
+      const long long w = (blockIdx.x + (long long)lt * gridDim.x) * TR + rr;
+      if (lt < myTiles && (!SMALL || rr < TR) && w < nwork) {
         o.live = true;
         o.frm = (int)(w / a.nlit);
         o.li = (int)(w - (long long)o.frm * a.nlit);
@@ -476,23 +485,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           ei[e] = puv[e] * sn;
         }
       }
-      store8<FMT, SPLIT>(Ehi, Elo, kmaj(r, pix0, ESZ, sboE), er);
-      store8<FMT, SPLIT>(Ehi, Elo, kmaj(r, ppr + pix0, ESZ, sboE), ei);
+      store8<FMT, SPLIT>(Ehi, Elo, kmaj(rf, pix0, ESZ, sboE), er);
+      store8<FMT, SPLIT>(Ehi, Elo, kmaj(rf, ppr + pix0, ESZ, sboE), ei);
     };
     const int ng8 = ppr / 8;
-    // the field of row R into (Ehi, Elo): this thread's pixel groups of
-    // parity h in [g0, g1) (two groups' loads in flight)
+    // the field of row R into (Ehi, Elo): this thread's pixel groups in
+    // [g0, g1) (two groups' loads in flight)
     auto build_field = [&](const Row& R, uint8_t* Ehi, uint8_t* Elo, int g0, int g1) {
       const int sy = R.sub / a.nsubx, sx = R.sub - sy * a.nsubx;
       const float* ph = a.phs + (long long)R.frm * a.phsFrameStride + (long long)sy * p * a.W + sx * p;
       const float* pu = a.pup + (long long)R.sub * pp;
-      for (int g8 = g0 + h; g8 < g1; g8 += 4) {
+      for (int g8 = g0 + part; g8 < g1; g8 += 2 * parts) {
         float phA[8], puA[8], phB[8], puB[8];
-        const bool two = g8 + 2 < g1;
+        const bool two = g8 + parts < g1;
         load_group(R, ph, pu, g8, phA, puA);
-        if (two) load_group(R, ph, pu, g8 + 2, phB, puB);
+        if (two) load_group(R, ph, pu, g8 + parts, phB, puB);
         emit_group(Ehi, Elo, R, g8, phA, puA);
-        if (two) emit_group(Ehi, Elo, R, g8 + 2, phB, puB);
+        if (two) emit_group(Ehi, Elo, R, g8 + parts, phB, puB);
       }
     };
     // with help the first tile's groups split at gMid (even): the field
@@ -500,14 +509,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const int gMid = (ng8 / 2) & ~1;
 
     {
-      // ---- field build (warps 8-15): row r, pixel groups of parity h.
+      // ---- field build (warps 8-15): row rf, its share of the pixel groups.
       // With help the epilogue warps run the first pass of this loop too
       // (one copy of the field code for both roles), then leave it.
-      Row next = row_of(0);
+      Row next = row_of(0, rf);
       const int fieldTiles = fieldRole ? myTiles : (help ? 1 : 0);
       for (int lt = 0; lt < fieldTiles; lt++) {
         const Row R = next;
-        if (fieldRole) next = row_of(lt + 1);  // its index loads overlap this tile
+        if (fieldRole) next = row_of(lt + 1, rf);  // its index loads overlap this tile
         const int eb = g.dbE ? (lt & 1) : 0;
         uint8_t* Ehi = A1hi + (size_t)eb * L.a1Half * (SPLIT ? 2 : 1);
         uint8_t* Elo = Ehi + L.a1Half;
@@ -516,8 +525,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         if (lt < reuse && fieldRole) {
           // zero K padding beyond 2*ppr once per buffer (none when 2*ppr is
           // a multiple of 16)
-          for (int k = 2 * ppr + h; k < g.K1; k += 2) {
-            const uint32_t off = kmaj(r, k, ESZ, sboE);
+          for (int k = 2 * ppr + part; k < g.K1; k += parts) {
+            const uint32_t off = kmaj(rf, k, ESZ, sboE);
             if constexpr (ESZ == 4) {
               *reinterpret_cast<uint32_t*>(Ehi + off) = 0u;
             } else {
@@ -558,7 +567,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const float skyv = nv.skyv;
         float* out = a.bimg + (long long)P.frm * a.bimgFrameStride + (long long)i * mm;
         const float* skyA = a.skyArr ? a.skyArr + (long long)i * mm : nullptr;
-        for (int cb = h * 32; cb < mm; cb += 64) {
+        for (int cb = h * 32; cb < mm && liveLanes; cb += 64) {
           uint32_t v[32];
           tc::tmem_ld32(tmem + d2c + lanebase + cb, v);
           tc::tmem_ld_wait();
@@ -606,7 +615,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             wait(&bars.a2free[0], (gA - 1) & 1);
           }
         };
-        if (g.CW == 64) {
+        if (!liveLanes) {
+          if (lane == 0) tc::mbar_arrive(&bars.d1free[d1b]);
+          a2_wait();
+        } else if (g.CW == 64) {
           float I[32];
           {
             // both halves in flight before one wait
@@ -678,12 +690,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       };
 
       Row prev{false, 0, 0, 0};
-      Row cur = row_of(0);
+      Row cur = row_of(0, r);
       RowNorm prevN{1.f, 0.f};
       RowNorm curN = row_norm(cur);
       float isc = (iscale && cur.live) ? iscale[cur.sub] : 1.f;
       for (int lt = 0; lt < myTiles; lt++) {
-        const Row next = row_of(lt + 1);
+        const Row next = row_of(lt + 1, r);
         const float iscn = (iscale && next.live) ? iscale[next.sub] : 1.f;
         const RowNorm nextN = row_norm(next);  // used two read-outs from now
         for (int oc = 0; oc < g.noc; oc++) {
@@ -760,16 +772,41 @@ void put_val(int fmt, bool split, uint8_t* hi, uint8_t* lo, uint32_t off, double
   }
 }
 
+// A launch whose tiles do not fill the SMs takes tiles of fewer live rows, so
+// that more SMs share its field build, phase loads and image stores (the
+// MMAs of a tile cost the same): 32 rows as long as every SM then has at most
+// one tile, then 64.  One tile per CTA needs no second field buffer; the W2
+// ring gets its shared memory.  One frame of the 74x74 sensor through host
+// arrays: 58.9 us with tiles of 128 rows (32 CTAs), 54.7 with 64, 53.4 with 32.
+GemmGeom small_launch(const GemmGeom& g0, long long nwork, int numSMs) {
+  GemmGeom g = g0;
+  g.TR = nwork <= 32LL * numSMs ? 32 : (nwork <= 64LL * numSMs ? 64 : kTileSubaps);
+  if (g.TR < kTileSubaps && g.dbE) {
+    GemmGeom t = g;
+    t.dbE = 0;
+    t.NK = 2;
+    t.NW = 0;
+    const GemmSmem base = gemm_smem_layout(t);
+    if (base.total <= kGemmSmemLimit) {
+      t.NW = std::min<int>(kGemmMaxNW, (int)((kGemmSmemLimit - base.total) / base.wStage));
+      if (t.NW > g.NW) g = t;
+    }
+  }
+  return g;
+}
+
 template <int FMT, int PASSES>
-cudaError_t launch_one(const WfsArgs& a, const GemmGeom& g, const float* iscale, int numSMs, int* err,
+cudaError_t launch_one(const WfsArgs& a, const GemmGeom& g0, const float* iscale, int numSMs, int* err,
                        cudaStream_t stream) {
-  const int smem = (int)gemm_smem_layout(g).total;
   const long long nwork = (long long)a.nlit * a.nframes;
-  const long long ntiles = (nwork + kTileSubaps - 1) / kTileSubaps;
+  const GemmGeom g = small_launch(g0, nwork, numSMs);
+  const int smem = (int)gemm_smem_layout(g).total;
+  const long long ntiles = (nwork + g.TR - 1) / g.TR;
   const int grid = (int)(ntiles < numSMs ? (ntiles > 0 ? ntiles : 1) : numSMs);
-  cudaError_t e = kernel_smem_setup((const void*)wfs_gemm_kernel<FMT, PASSES>, smem, kGemmThreads, nullptr);
+  auto kern = g.TR < kTileSubaps ? wfs_gemm_kernel<FMT, PASSES, true> : wfs_gemm_kernel<FMT, PASSES, false>;
+  cudaError_t e = kernel_smem_setup((const void*)kern, smem, kGemmThreads, nullptr);
   if (e != cudaSuccess) return e;
-  wfs_gemm_kernel<FMT, PASSES><<<grid, kGemmThreads, smem, stream>>>(a, g, iscale, err);
+  kern<<<grid, kGemmThreads, smem, stream>>>(a, g, iscale, err);
   return cudaGetLastError();
 }
 
@@ -801,8 +838,7 @@ std::vector<int> chunk_widths(int cc, int N2) {
 std::vector<GemmGeom> stagings_of_width(GemmGeom g, int cw, int cc, int passes) {
   std::vector<GemmGeom> out;
   const int esz = g.fmt == kFmtTF32 ? 4 : 2;
-  // dynamic limit: 227 KB minus the kernel's static shared memory (< 4 KB)
-  const uint32_t limit = 227 * 1024 - 4096;
+  const uint32_t limit = kGemmSmemLimit;
   g.CW = cw;
   g.noc = (cc + cw - 1) / cw;
   g.nd1 = (cw == 64 && g.N2 <= 128) ? 3 : 2;

@@ -238,12 +238,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   if (warp == kConsumers / 32) {
     // ================= GEMM1 producer (MMA issue only) =================
-    // The whole warp runs the loop (so that counters and descriptors stay
-    // warp-uniform); lane 0 issues the MMAs and commits.  W2 chunk gJ sits
+    // The whole warp runs the loop, so that counters and descriptors stay
+    // warp-uniform; one elected lane issues the MMAs and commits.  W2 chunk gJ sits
     // in ring stage cs with phase bit cph (the loader warp fills the ring);
     // output chunk gC goes to D1 buffer d1b in round d1r.
     if (myTiles > 0) {
-      const bool leader = lane == 0;
       const uint32_t idesc1 = tc::idesc_f32acc(FMT, 128, 2 * g.CW);
       const uint32_t wbase = tc::smem_addr(smem + L.w);
       // descriptors: the 14-bit start-address field (bits 0-13, in 16-byte
@@ -275,30 +274,28 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             wait(&bars.wfull[cs], cph);
             const uint64_t dWh = dW0 + (uint64_t)cs * dWstage;
             const int ks1 = min(K1B, (kc + 1) * g.KCB) >> 5;
-            if (leader) {
-              for (uint64_t wo = 0; ks < ks1; ks++, wo += 16) {
-                const uint64_t eo = (uint64_t)ks * 16;
-                tc::mma<FMT>(dcol, dEh + eo, dWh + wo, idesc1, ks > 0 ? 1u : 0u);
-                if constexpr (SPLIT) {
-                  tc::mma<FMT>(dcol, dEh + eo, dWh + dWlo + wo, idesc1, 1u);
-                  tc::mma<FMT>(dcol, dEl + eo, dWh + wo, idesc1, 1u);
-                }
+            __syncwarp();
+            for (uint64_t wo = 0; ks < ks1; ks++, wo += 16) {
+              const uint64_t eo = (uint64_t)ks * 16;
+              tc::mma<FMT>(dcol, dEh + eo, dWh + wo, idesc1, ks > 0 ? 1u : 0u);
+              if constexpr (SPLIT) {
+                tc::mma<FMT>(dcol, dEh + eo, dWh + dWlo + wo, idesc1, 1u);
+                tc::mma<FMT>(dcol, dEl + eo, dWh + wo, idesc1, 1u);
               }
-              tc::mma_commit(&bars.wfree[cs]);
             }
-            ks = ks1;
+            tc::mma_commit(&bars.wfree[cs]);
             if (++cs == g.NW) {
               cs = 0;
               cph ^= 1u;
             }
           }
-          if (leader) tc::mma_commit(&bars.d1full[d1b]);
+          tc::mma_commit(&bars.d1full[d1b]);
           if (++d1b == g.nd1) {
             d1b = 0;
             d1r++;
           }
         }
-        if (leader) tc::mma_commit(&bars.efree[eb]);
+        tc::mma_commit(&bars.efree[eb]);
       }
     }
     __syncwarp();
@@ -325,7 +322,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     __syncwarp();
   } else if (warp == kConsumers / 32 + 1) {
-    // ================= GEMM2 producer (whole warp, lane 0 issues) =================
+    // ================= GEMM2 producer (whole warp, one lane issues) =================
     if (myTiles > 0) {
       const bool leader = lane == 0;
       const int totalK = myTiles * g.noc;
@@ -362,20 +359,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           wait(&bars.kfull[ksg], kph);
           tc::fence_after_sync();
           const uint64_t dKh = dK0 + (uint64_t)ksg * dKstage;
-          if (leader) {
-            for (int ks = 0; ks < ks2; ks++) {
-              const uint64_t o = (uint64_t)ks * 16;
-              const uint32_t acc0 = (oc > 0 || ks > 0) ? 1u : 0u;
-              tc::mma<FMT>(dcol, dAh + o, dKh + o, idesc2, acc0);
-              if constexpr (SPLIT) {
-                tc::mma<FMT>(dcol, dAh + o, dKh + dKlo + o, idesc2, 1u);
-                tc::mma<FMT>(dcol, dAl + o, dKh + o, idesc2, 1u);
-              }
+          __syncwarp();
+          for (int ks = 0; ks < ks2; ks++) {
+            const uint64_t o = (uint64_t)ks * 16;
+            const uint32_t acc0 = (oc > 0 || ks > 0) ? 1u : 0u;
+            tc::mma<FMT>(dcol, dAh + o, dKh + o, idesc2, acc0);
+            if constexpr (SPLIT) {
+              tc::mma<FMT>(dcol, dAh + o, dKh + dKlo + o, idesc2, 1u);
+              tc::mma<FMT>(dcol, dAl + o, dKh + o, idesc2, 1u);
             }
-            tc::mma_commit(&bars.a2free[ab]);
-            tc::mma_commit(&bars.kfree[ksg]);
-            if (oc == g.noc - 1) tc::mma_commit(&bars.d2full);
           }
+          tc::mma_commit(&bars.a2free[ab]);
+          tc::mma_commit(&bars.kfree[ksg]);
+          if (oc == g.noc - 1) tc::mma_commit(&bars.d2full);
           if (nextK < totalK) {
             wait(&bars.kfree[ksg], kph);
             kload(ksg);

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const long long w = (blockIdx.x + (long long)lt * gridDim.x) * TR + rr;
       if (lt < myTiles && (!SMALL || rr < TR) && w < nwork) {
         o.live = true;
-        o.frm = (int)(w / a.nlit);
+        o.frm = nwork <= 0x7fffffffLL ? (int)((unsigned)w / (unsigned)a.nlit) : (int)(w / a.nlit);
         o.li = (int)(w - (long long)o.frm * a.nlit);
         o.sub = a.lit[o.li];
       }
@@ -542,19 +542,26 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       // ---- epilogue ----
       int d1b = 0;
       uint32_t d1r = 0, gA = 0;
-      // binned image of tile lt (row P) from D2: normalise, sky -> bimg
-      // per-row image scale and sky level, computed a tile before their D2
-      // read-out so the scattered loads are off the read-out's critical path
+      // per-row image scale and sky level: their scattered loads are issued a
+      // tile ahead, once the row is known, and used at the end of that tile
+      // (loaded and divided at once they held each tile up by two dependent
+      // global loads: 5 of 25 thousand cycles)
+      struct RowRaw {
+        float totsig, frac, sig, isc;
+      };
       struct RowNorm {
         float scale, skyv;
       };
-      auto row_norm = [&](const Row& P) {
+      auto row_raw = [&](const Row& P) {
         const int i = P.sub;
-        const float totsig = a.totsig[i], fr = a.frac[i];
-        float scale = totsig > 0.f ? (a.sigArr ? a.sigArr[i] / totsig : a.sig * fr / totsig) : 1.f;
-        if (iscale) scale = scale / iscale[i];  // undo the fp16 range scaling
-        return RowNorm{scale, a.sky * fr};
+        return RowRaw{a.totsig[i], a.frac[i], a.sigArr ? a.sigArr[i] : 0.f, iscale ? iscale[i] : 1.f};
       };
+      auto row_norm = [&](const RowRaw& v) {
+        float scale = v.totsig > 0.f ? (a.sigArr ? v.sig / v.totsig : a.sig * v.frac / v.totsig) : 1.f;
+        if (iscale) scale = scale / v.isc;  // undo the fp16 range scaling
+        return RowNorm{scale, a.sky * v.frac};
+      };
+      // binned image of tile lt (row P) from D2: normalise, sky -> bimg
       auto read_D2 = [&](int lt, const Row& P, const RowNorm& nv) {
         const int i = P.sub;
         wait(&bars.d2full, lt & 1);
@@ -686,14 +693,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       };
 
       Row prev{false, 0, 0, 0};
-      Row cur = row_of(0, r);
-      RowNorm prevN{1.f, 0.f};
-      RowNorm curN = row_norm(cur);
-      float isc = (iscale && cur.live) ? iscale[cur.sub] : 1.f;
+      Row cur = row_of(0, r), next = row_of(1, r);
+      RowRaw raw = row_raw(cur);
+      float isc = cur.live ? raw.isc : 1.f;  // 1 without range scaling
+      RowNorm prevN{1.f, 0.f}, curN = row_norm(raw);
       for (int lt = 0; lt < myTiles; lt++) {
-        const Row next = row_of(lt + 1, r);
-        const float iscn = (iscale && next.live) ? iscale[next.sub] : 1.f;
-        const RowNorm nextN = row_norm(next);  // used two read-outs from now
+        raw = row_raw(next);                   // the next tile's values
+        const Row after = row_of(lt + 2, r);  // and the row of the one after
         for (int oc = 0; oc < g.noc; oc++) {
           if (oc == 0 && lt >= 1) read_D2(lt - 1, prev, prevN);
           chunk(isc);
@@ -701,8 +707,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         prev = cur;
         prevN = curN;
         cur = next;
-        curN = nextN;
-        isc = iscn;
+        curN = row_norm(raw);
+        isc = cur.live ? raw.isc : 1.f;
+        next = after;
       }
       if (myTiles > 0) read_D2(myTiles - 1, prev, prevN);
     }

@@ -854,6 +854,7 @@ const FormEntry* form_entry(const shwfs_handle* h) {
   if (h->psfDim) {
     if (h->psfsize != N || h->padded != N || h->preBin > 1 || h->clipsize != N) return nullptr;
     if (2 * h->nimg == N) F = 2;
+    if (4 * h->nimg == N) F = 4;
   } else if (h->clipsize > N) {
     return nullptr;
   }

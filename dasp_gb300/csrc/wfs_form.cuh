@@ -29,10 +29,10 @@
 // indices rotated.  The DC and Nyquist columns of a row-transformed real
 // image are real and share one complex column (PACK below), which makes N/2
 // columns of N/2 + 1 and N/2 slots per lane group in every stage.  When the
-// image bins two by two (F = 2), the product with the PSF spectrum is
-// multiplied by the response of the sum of two pixels and folded to N/2
-// frequencies per axis, so that the inverse transforms are of half the size
-// and give the binned image.
+// image bins F by F pixels, F = 2 or 4, the product with the PSF spectrum is
+// multiplied by the response of the sum of F pixels and folded to N/F
+// frequencies per axis, so that the inverse transforms are of that size and
+// give the binned image.
 //
 // Even N, with no PSF or an N x N PSF, no pre-binning, phase-only input, no
 // optical binning (form_covers); everything else takes the block form.
@@ -153,20 +153,23 @@ __host__ __device__ inline int form_const_floats(int N, int P, int p, int C, int
 }
 constexpr int kFormWarps = 4;
 
-// 1 + exp(2 pi i k / N): the response of the sum of two neighbouring pixels
-template <int N>
-__host__ __device__ constexpr float2 pair_response(int k) {
-  const CS c = cos_sin_frac(k, N);
-  return float2{(float)(1.0 + c.c), (float)c.s};
-}
-template <int N>
-struct PairTable {
+// sum of exp(2 pi i j k / N) over j < F: the response of the sum of F pixels
+template <int N, int F>
+struct BinTable {
   float2 v[N];
 };
-template <int N>
-__host__ __device__ constexpr PairTable<N> make_pair_table() {
-  PairTable<N> t{};
-  for (int k = 0; k < N; k++) t.v[k] = pair_response<N>(k);
+template <int N, int F>
+__host__ __device__ constexpr BinTable<N, F> make_bin_table() {
+  BinTable<N, F> t{};
+  for (int k = 0; k < N; k++) {
+    double c = 0.0, s = 0.0;
+    for (int j = 0; j < F; j++) {
+      const CS e = cos_sin_frac(j * k % N, N);
+      c += e.c;
+      s += e.s;
+    }
+    t.v[k] = float2{(float)c, (float)s};
+  }
   return t;
 }
 
@@ -175,7 +178,7 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
   using G = FormGeom<N>;
   constexpr int H = G::H, ZS = G::ZS;
   constexpr int M = N / F;  // size of the inverse transforms
-  constexpr PairTable<N> kPair = make_pair_table<N>();
+  constexpr BinTable<N, F> kBin = make_bin_table<N, F>();
   static_assert(P == 0 || P == N, "the PSF has the FFT's size");
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
@@ -252,6 +255,7 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
 
   const bool storePre = a.mode & kStorePreNoise;
   const int rofs = P > 0 ? 1 : (N - (N - C) / 2 - C + 1) % N;  // image row i is |F|^2 row (i + rofs) mod N
+  const int whole = C % m == 0 ? C / m : 0;  // pixels binned per axis, 0 when fractional
   const float inv_mm = 1.0f / (float)mm, inv_m = 1.0f / (float)m, inv_nc = 1.0f / (float)ncen;
   const long long nwork = (long long)a.nlit * a.nframes;
   const long long ngroups = (nwork + S - 1) / S;
@@ -380,12 +384,11 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
           }
         }
         float2 v[M];
-        if constexpr (F == 2) {
 #pragma unroll
-          for (int k = 0; k < M; k++) v[k] = cadd(cmul(y[k], kPair.v[k]), cmul(y[k + M], kPair.v[k + M]));
-        } else {
+        for (int k = 0; k < M; k++) {
+          v[k] = F == 1 ? y[k] : cmul(y[k], kBin.v[k]);
 #pragma unroll
-          for (int k = 0; k < M; k++) v[k] = y[k];
+          for (int f = 1; f < F; f++) v[k] = cadd(v[k], cmul(y[k + f * M], kBin.v[k + f * M]));
         }
         fft<M, 1, N>(v);
 #pragma unroll
@@ -399,13 +402,21 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
         const bool two = 2 * lq + 1 < M;
         float2 z[M];
         const float2 x0 = r[0], y0 = two ? r[H] : make_float2(0.f, 0.f);
-        if constexpr (F == 2) {
-          z[0] = make_float2(2.f * x0.x, 2.f * y0.x);
+        if constexpr (F > 1) {
+          // frequency i of the real row whose entries start at o
+          auto at = [&](int o, int i) {
+            return i == H ? make_float2(o ? y0.y : x0.y, 0.f) : (i < H ? r[o + i] : cconj(r[o + N - i]));
+          };
+          z[0] = make_float2(F * x0.x, F * y0.x);
 #pragma unroll
           for (int l = 1; l <= M / 2; l++) {
-            const float2 bl = kPair.v[l], bm = kPair.v[l + M];
-            const float2 X = cadd(cmul(r[l], bl), cmul(cconj(r[M - l]), bm));
-            const float2 Y = two ? cadd(cmul(r[H + l], bl), cmul(cconj(r[H + M - l]), bm)) : make_float2(0.f, 0.f);
+            float2 X = make_float2(0.f, 0.f), Y = X;
+#pragma unroll
+            for (int f = 0; f < F; f++) {
+              const float2 bf = kBin.v[l + f * M];
+              X = f == 0 ? cmul(at(0, l), bf) : cadd(X, cmul(at(0, l + f * M), bf));
+              if (two) Y = f == 0 ? cmul(at(H, l), bf) : cadd(Y, cmul(at(H, l + f * M), bf));
+            }
             if (2 * l == M) {
               z[l] = make_float2(X.x, Y.x);
             } else {
@@ -435,7 +446,7 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
     for (int w = lane; w < ns * mm; w += 32) {
       const int s = div_small(w, mm, inv_mm), pix = w - s * mm;
       int I, J;
-      if constexpr (F == 2) {
+      if constexpr (F > 1) {
         I = pix / M;
         J = pix - I * M;
       } else {
@@ -453,10 +464,14 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
         return z[2 * ((i >> 1) * ZS + j) + (i & 1)];
       };
       float v;
-      if (F == 2 || C == m) {
+      if (F > 1 || C == m) {
         v = at(I, J);
-      } else if (C == 2 * m) {
+      } else if (whole == 2) {
         v = at(2 * I, 2 * J) + at(2 * I, 2 * J + 1) + at(2 * I + 1, 2 * J) + at(2 * I + 1, 2 * J + 1);
+      } else if (whole) {
+        v = 0.f;
+        for (int i = whole * I; i < whole * (I + 1); i++)
+          for (int j = whole * J; j < whole * (J + 1); j++) v += at(i, j);
       } else {
         v = 0.f;
         const int ilo = s_binLo[I], ihi = s_binHi[I], jlo = s_binLo[J], jhi = s_binHi[J];
@@ -574,7 +589,8 @@ struct FormEntry {
   cudaError_t (*launch_multi)(const FormMulti& m, int threads, int smem, cudaStream_t);
   cudaError_t (*occupancy_multi)(int* ctas_per_sm, int threads, int smem);
 };
-// (fftsize, 0 without a spot PSF else fftsize, pixels binned per axis: 1 or 2)
+// (fftsize, 0 without a spot PSF else fftsize, pixels binned per axis in the
+// transforms: 1, 2 or 4)
 using FormKey = std::array<int, 3>;
 inline std::map<FormKey, FormEntry>& form_registry() {
   static std::map<FormKey, FormEntry> r;
@@ -608,10 +624,13 @@ struct FormRegistrar {
 };
 
 // fftsize N without a PSF, with an N x N PSF, and with one and images of N / 2
-// pixels
-#define SHWFS_REGISTER_FORM(N)                            \
+// pixels; SHWFS_REGISTER_FORM4 (N a multiple of 4): of N / 4 pixels too
+#define SHWFS_REGISTER_FORM(N)                               \
   static ::shwfs::FormRegistrar<N, 0, 1> shwfs_form_##N##_0; \
   static ::shwfs::FormRegistrar<N, N, 1> shwfs_form_##N##_1; \
   static ::shwfs::FormRegistrar<N, N, 2> shwfs_form_##N##_2;
+#define SHWFS_REGISTER_FORM4(N) \
+  SHWFS_REGISTER_FORM(N)        \
+  static ::shwfs::FormRegistrar<N, N, 4> shwfs_form_##N##_4;
 
 }  // namespace shwfs

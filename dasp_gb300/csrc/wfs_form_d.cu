@@ -2,5 +2,5 @@
 #include "wfs_form.cuh"
 
 SHWFS_REGISTER_FORM(50)
-SHWFS_REGISTER_FORM(60)
-SHWFS_REGISTER_FORM(64)
+SHWFS_REGISTER_FORM4(60)
+SHWFS_REGISTER_FORM4(64)

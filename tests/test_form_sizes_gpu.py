@@ -38,11 +38,11 @@ def _check(c, frames=1):
 
 @pytest.mark.parametrize("N", SIZES)
 @pytest.mark.parametrize("psf", [None, "gauss", "gauss4d"])
-@pytest.mark.parametrize("images", ["half", "full", "ragged"])
+@pytest.mark.parametrize("images", ["half", "quarter", "full", "ragged"])
 def test_every_size(N, psf, images):
-    # images of half the FFT (folded transforms with a PSF), of all of it and
-    # of a width that bins fractionally
-    m = {"half": N // 2, "full": N, "ragged": N // 2 - 1}[images]
+    # images of half and a quarter of the FFT (folded transforms with a PSF),
+    # of all of it and of a width that bins fractionally
+    m = {"half": N // 2, "quarter": N // 4, "full": N, "ragged": N // 2 - 1}[images]
     c = Case(nsubx=5, p=N // 2, N=N, C=N, m=m, ncen=m, psf=psf, sig=1e4, skybrightness=2.0, noiseFloor=1.0,
              phase_seed=N, L0=2.0)
     _check(c)

@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kFinishThreads)
 // keeps up to kScratchKeep bytes across synchronisations.  The device's
 // default pool gives its memory back at every synchronisation, and a call
 // after one then waited about 200 us for it to be mapped again.
-constexpr uint64_t kScratchKeep = 4u << 20;
+constexpr uint64_t kScratchKeep = 64u << 20;
 struct ScratchPool {
   cudaMemPool_t pool = nullptr;
   int users = 0;

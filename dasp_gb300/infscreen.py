@@ -201,19 +201,19 @@ def pupil_phase(layers, pupil, out, pupil_area=None, wavelength=500.0, remove_pi
     from . import _lib
     n = len(layers)
     npup = int(out.shape[-1])
+    square = (npup, npup)
     for t in (pupil, out):
-        if not (t.is_cuda and t.is_contiguous() and str(t.dtype) == "torch.float32" and tuple(t.shape) == (npup, npup)):
+        if not (t.is_cuda and t.shape == square and t.is_contiguous() and t.dtype.is_floating_point
+                and t.element_size() == 4):
             raise ValueError("pupil and out must be npup x npup contiguous float32 CUDA tensors")
     if pupil_area is None:
-        pupil_area = float(pupil.double().sum().item())
-    arr_s = (ctypes.c_void_p * n)(*[ly[0]._s.value for ly in layers])
-    y0 = (ctypes.c_int * n)(*[int(ly[1]) for ly in layers])
-    x0 = (ctypes.c_int * n)(*[int(ly[2]) for ly in layers])
-    ys = (ctypes.c_float * n)(*[float(ly[3]) for ly in layers])
-    xs = (ctypes.c_float * n)(*[float(ly[4]) for ly in layers])
+        pupil_area = pupil.double().sum().item()
+    screens, y0, x0, ys, xs = list(zip(*layers))[:5]
+    ints, floats = ctypes.c_int * n, ctypes.c_float * n
     s = getattr(stream, "cuda_stream", stream)
-    _lib.check(_lib.lib().shwfs_screens_pupil_phase(arr_s, n, y0, x0, ys, xs, npup, pupil.data_ptr(),
-                                                    float(pupil_area), 1 if remove_piston else 0,
-                                                    float(500.0 / wavelength), out.data_ptr(), s),
-               "screens_pupil_phase")
+    _lib.check(_lib.lib().shwfs_screens_pupil_phase((ctypes.c_void_p * n)(*[scr._s.value for scr in screens]), n,
+                                                    ints(*map(int, y0)), ints(*map(int, x0)), floats(*map(float, ys)),
+                                                    floats(*map(float, xs)), npup, pupil.data_ptr(), float(pupil_area),
+                                                    1 if remove_piston else 0, float(500.0 / wavelength),
+                                                    out.data_ptr(), s), "screens_pupil_phase")
     return out

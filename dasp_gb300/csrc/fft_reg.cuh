@@ -128,6 +128,57 @@ __host__ __device__ __forceinline__ float2 cscale(float2 a, float s) { return ma
 __host__ __device__ __forceinline__ float2 cmuli(float2 a) { return make_float2(-a.y, a.x); }
 __host__ __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 
+// Packed pairs of float operations for the butterflies: one instruction for
+// both parts of a complex sum (the transforms are bound by instruction issue).
+#if defined(__CUDA_ARCH__)
+#define SHWFS_F32X2(op, r, a, b)                                                                                   \
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t" op                             \
+      ".rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"                                                            \
+      : "=f"(r.x), "=f"(r.y)                                                                                       \
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y))
+#endif
+__host__ __device__ __forceinline__ float2 padd(float2 a, float2 b) {
+#if defined(__CUDA_ARCH__)
+  float2 r;
+  SHWFS_F32X2("add", r, a, b);
+  return r;
+#else
+  return cadd(a, b);
+#endif
+}
+__host__ __device__ __forceinline__ float2 psub(float2 a, float2 b) {
+#if defined(__CUDA_ARCH__)
+  float2 r;
+  SHWFS_F32X2("sub", r, a, b);
+  return r;
+#else
+  return csub(a, b);
+#endif
+}
+// c * a
+__host__ __device__ __forceinline__ float2 pmul(float c, float2 a) {
+#if defined(__CUDA_ARCH__)
+  float2 r, k = make_float2(c, c);
+  SHWFS_F32X2("mul", r, k, a);
+  return r;
+#else
+  return cscale(a, c);
+#endif
+}
+// c * a + b
+__host__ __device__ __forceinline__ float2 pfma(float c, float2 a, float2 b) {
+#if defined(__CUDA_ARCH__)
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %2};\n\tmov.b64 y, {%3, %4};\n\tmov.b64 z, {%5, %6};\n\t"
+      "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(c), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+#else
+  return make_float2(c * a.x + b.x, c * a.y + b.y);
+#endif
+}
+
 __host__ __device__ constexpr int first_radix(int N) {
   return (N % 4 == 0 && N != 8) ? 4 : (N % 2 == 0 ? 2 : (N % 3 == 0 ? 3 : 5));
 }
@@ -139,25 +190,25 @@ __host__ __device__ __forceinline__ void butterfly(float2 (&a)[R]);
 template <>
 __host__ __device__ __forceinline__ void butterfly<2, -1>(float2 (&a)[2]) {
   float2 t = a[0];
-  a[0] = cadd(t, a[1]);
-  a[1] = csub(t, a[1]);
+  a[0] = padd(t, a[1]);
+  a[1] = psub(t, a[1]);
 }
 template <>
 __host__ __device__ __forceinline__ void butterfly<2, 1>(float2 (&a)[2]) {
   float2 t = a[0];
-  a[0] = cadd(t, a[1]);
-  a[1] = csub(t, a[1]);
+  a[0] = padd(t, a[1]);
+  a[1] = psub(t, a[1]);
 }
 
 template <int S>
 __host__ __device__ __forceinline__ void bfly4(float2 (&a)[4]) {
-  float2 s02 = cadd(a[0], a[2]), d02 = csub(a[0], a[2]);
-  float2 s13 = cadd(a[1], a[3]), d13 = csub(a[1], a[3]);
+  float2 s02 = padd(a[0], a[2]), d02 = psub(a[0], a[2]);
+  float2 s13 = padd(a[1], a[3]), d13 = psub(a[1], a[3]);
   // w = exp(S*i*pi/2) = S*i
   float2 id13 = cmuli(d13);
   if (S < 0) id13 = make_float2(-id13.x, -id13.y);
-  a[0] = cadd(s02, s13);
-  a[2] = csub(s02, s13);
+  a[0] = padd(s02, s13);
+  a[2] = psub(s02, s13);
   a[1] = cadd(d02, id13);
   a[3] = csub(d02, id13);
 }
@@ -188,13 +239,12 @@ __host__ __device__ __forceinline__ void bfly5(float2 (&a)[5]) {
   constexpr float c2 = -0.809016994374947424f;  // cos(4*pi/5)
   constexpr float s1 = 0.951056516295153572f;   // sin(2*pi/5)
   constexpr float s2 = 0.587785252292473129f;   // sin(4*pi/5)
-  float2 t1 = cadd(a[1], a[4]), t3 = csub(a[1], a[4]);
-  float2 t2 = cadd(a[2], a[3]), t4 = csub(a[2], a[3]);
-  float2 b1 = make_float2(a[0].x + c1 * t1.x + c2 * t2.x, a[0].y + c1 * t1.y + c2 * t2.y);
-  float2 b2 = make_float2(a[0].x + c2 * t1.x + c1 * t2.x, a[0].y + c2 * t1.y + c1 * t2.y);
-  float2 d1 = cscale(cmuli(make_float2(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y)), (float)S);
-  float2 d2 = cscale(cmuli(make_float2(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y)), (float)S);
-  a[0] = cadd(a[0], cadd(t1, t2));
+  const float2 t1 = padd(a[1], a[4]), t3 = psub(a[1], a[4]);
+  const float2 t2 = padd(a[2], a[3]), t4 = psub(a[2], a[3]);
+  const float2 b1 = pfma(c2, t2, pfma(c1, t1, a[0])), b2 = pfma(c1, t2, pfma(c2, t1, a[0]));
+  const float2 d1 = cscale(cmuli(pfma(s2, t4, pmul(s1, t3))), (float)S);
+  const float2 d2 = cscale(cmuli(pfma(-s1, t4, pmul(s2, t3))), (float)S);
+  a[0] = padd(a[0], padd(t1, t2));
   a[1] = cadd(b1, d1);
   a[4] = csub(b1, d1);
   a[2] = cadd(b2, d2);

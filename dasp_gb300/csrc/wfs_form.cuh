@@ -20,8 +20,9 @@
 // 74x74 sensor, 30 us at the nominal FP32 rate and 8 us of memory time).  The
 // block form (wfs_plain.cuh), which keeps 128 threads in step over uneven
 // stages and transforms the zero inputs and the unbinned image too, took 341
-// us there, this one 129; one frame of the 74x74 LGS sensor (fftsize 32, a PSF
-// per subaperture) 114 and 29 us, one 8x8 frame through host arrays 32 and 17.
+// us there, this one 121 (130 with scalar butterflies and five CTAs per SM at
+// 20 points); one frame of the 74x74 LGS sensor (fftsize 32, a PSF per
+// subaperture) 114 and 27 us, one 8x8 frame through host arrays 32 and 17.
 //
 // The field is conjugated because |DFT(conj E)|^2 at u is |DFT(E)|^2 at N - u:
 // the 180-degree rotation of the power spectrum (addPowerSpecCentral) is then
@@ -63,31 +64,26 @@ __device__ __forceinline__ void butterfly_nz(float2 (&a)[R]) {
   } else if constexpr (R == 4) {  // NZ == 2 or 3
     float2 i1 = cmuli(a[1]);
     if (S < 0) i1 = make_float2(-i1.x, -i1.y);
-    const float2 s = NZ == 3 ? cadd(a[0], a[2]) : a[0], d = NZ == 3 ? csub(a[0], a[2]) : a[0], b = a[1];
-    a[0] = cadd(s, b);
-    a[2] = csub(s, b);
+    const float2 s = NZ == 3 ? padd(a[0], a[2]) : a[0], d = NZ == 3 ? psub(a[0], a[2]) : a[0], b = a[1];
+    a[0] = padd(s, b);
+    a[2] = psub(s, b);
     a[1] = cadd(d, i1);
     a[3] = csub(d, i1);
   } else {  // R == 5, NZ == 2, 3 or 4
     constexpr float c1 = 0.309016994374947424f, c2 = -0.809016994374947424f;  // cos(2 pi / 5), cos(4 pi / 5)
     constexpr float s1 = 0.951056516295153572f, s2 = 0.587785252292473129f;   // sin(2 pi / 5), sin(4 pi / 5)
-    const float2 z = make_float2(0.f, 0.f);
-    const float2 x0 = a[0], x1 = a[1], x2 = NZ > 2 ? a[2] : z, x3 = NZ > 3 ? a[3] : z;
-    const float2 t2 = NZ > 3 ? cadd(x2, x3) : x2, t4 = NZ > 3 ? csub(x2, x3) : x2;
-    float2 b1, b2, d1, d2;
+    const float2 x0 = a[0], x1 = a[1], x2 = a[2], x3 = a[3];
+    float2 b1 = pfma(c1, x1, x0), b2 = pfma(c2, x1, x0), e1 = pmul(s1, x1), e2 = pmul(s2, x1);
+    a[0] = padd(x0, x1);
     if constexpr (NZ > 2) {
-      b1 = make_float2(x0.x + c1 * x1.x + c2 * t2.x, x0.y + c1 * x1.y + c2 * t2.y);
-      b2 = make_float2(x0.x + c2 * x1.x + c1 * t2.x, x0.y + c2 * x1.y + c1 * t2.y);
-      d1 = cscale(cmuli(make_float2(s1 * x1.x + s2 * t4.x, s1 * x1.y + s2 * t4.y)), (float)S);
-      d2 = cscale(cmuli(make_float2(s2 * x1.x - s1 * t4.x, s2 * x1.y - s1 * t4.y)), (float)S);
-      a[0] = cadd(x0, cadd(x1, t2));
-    } else {
-      b1 = make_float2(x0.x + c1 * x1.x, x0.y + c1 * x1.y);
-      b2 = make_float2(x0.x + c2 * x1.x, x0.y + c2 * x1.y);
-      d1 = cscale(cmuli(make_float2(s1 * x1.x, s1 * x1.y)), (float)S);
-      d2 = cscale(cmuli(make_float2(s2 * x1.x, s2 * x1.y)), (float)S);
-      a[0] = cadd(x0, x1);
+      const float2 t2 = NZ > 3 ? padd(x2, x3) : x2, t4 = NZ > 3 ? psub(x2, x3) : x2;
+      b1 = pfma(c2, t2, b1);
+      b2 = pfma(c1, t2, b2);
+      e1 = pfma(s2, t4, e1);
+      e2 = pfma(-s1, t4, e2);
+      a[0] = padd(a[0], t2);
     }
+    const float2 d1 = cscale(cmuli(e1), (float)S), d2 = cscale(cmuli(e2), (float)S);
     a[1] = cadd(b1, d1);
     a[4] = csub(b1, d1);
     a[2] = cadd(b2, d2);
@@ -256,7 +252,7 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
   const bool storePre = a.mode & kStorePreNoise;
   const int rofs = P > 0 ? 1 : (N - (N - C) / 2 - C + 1) % N;  // image row i is |F|^2 row (i + rofs) mod N
   const int whole = C % m == 0 ? C / m : 0;  // pixels binned per axis, 0 when fractional
-  const float inv_mm = 1.0f / (float)mm, inv_m = 1.0f / (float)m, inv_nc = 1.0f / (float)ncen;
+  const float inv_m = 1.0f / (float)m, inv_nc = 1.0f / (float)ncen;
   const long long nwork = (long long)a.nlit * a.nframes;
   const long long ngroups = (nwork + S - 1) / S;
   for (long long g = warp0; g < ngroups; g += nwarps) {
@@ -365,10 +361,11 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
 #pragma unroll
         for (int k = 0; k <= H; k++) {
           const int n = (N - k) % N;
-          float2 ak = psf[k * HS + lq], an = psf[n * HS + lq];
+          float2 ak = psf[k * HS + lq], an = psf[n * HS + lq], bk, bn;
           const float2 yk = y[k], yn = y[n];
           if (lq == 0) {
-            float2 bk = psf[k * HS + H], bn = psf[n * HS + H];
+            bk = psf[k * HS + H];
+            bn = psf[n * HS + H];
             if (!psf2d) {
               const float2 dk = ak, dn = an;
               ak = make_float2(0.5f * (dk.x + bk.x), 0.5f * (dk.y + bk.y));
@@ -376,11 +373,12 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
               an = make_float2(0.5f * (dn.x + bn.x), 0.5f * (dn.y + bn.y));
               bn = make_float2(0.5f * (dn.x - bn.x), 0.5f * (dn.y - bn.y));
             }
-            y[k] = cadd(cmul(ak, yk), cmul(bk, cconj(yn)));
-            if (n != k) y[n] = cadd(cmul(an, yn), cmul(bn, cconj(yk)));
-          } else {
-            y[k] = cmul(ak, yk);
-            if (n != k) y[n] = cmul(an, yn);
+          }
+          y[k] = cmul(ak, yk);
+          if (n != k) y[n] = cmul(an, yn);
+          if (lq == 0) {
+            y[k] = cadd(y[k], cmul(bk, cconj(yn)));
+            if (n != k) y[n] = cadd(y[n], cmul(bn, cconj(yk)));
           }
         }
         float2 v[M];
@@ -443,8 +441,18 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
 
     // ---- 5: bin, normalise, sky [threshold, power] -> bimg ----
     const float* zf = reinterpret_cast<const float*>(zb);
+    int s5 = 0, pix5 = lane;
+    while (pix5 >= mm) {
+      pix5 -= mm;
+      s5++;
+    }
     for (int w = lane; w < ns * mm; w += 32) {
-      const int s = div_small(w, mm, inv_mm), pix = w - s * mm;
+      const int s = s5, pix = pix5;
+      pix5 += 32;
+      while (pix5 >= mm) {
+        pix5 -= mm;
+        s5++;
+      }
       int I, J;
       if constexpr (F > 1) {
         I = pix / M;
@@ -552,9 +560,11 @@ __device__ __forceinline__ void form_body(const WfsArgs& a, long long warp0, lon
   }
 }
 
+// CTAs per SM that the registers are cut for: the most that do not spill in the
+// form's main variants (20 points: six at 80 registers 122 us, five 125).
 template <int N>
 constexpr int form_min_blocks() {
-  return N <= 24 ? 5 : (N <= 32 ? 4 : 2);
+  return N <= 20 ? 6 : (N <= 24 ? 5 : (N <= 32 ? 4 : 2));
 }
 template <int N, int P, int F>
 __global__ void __launch_bounds__(32 * kFormWarps, form_min_blocks<N>()) wfs_form_kernel(const __grid_constant__ WfsArgs a) {

@@ -100,6 +100,20 @@ __device__ __forceinline__ float dec(uint32_t b) {
   }
 }
 
+// two elements in one conversion, x0 in the low half (16-bit formats)
+template <int FMT>
+__device__ __forceinline__ uint32_t enc2(float x0, float x1) {
+  uint32_t r;
+  if constexpr (FMT == kFmtBF16) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(x0, x1);
+    memcpy(&r, &v, 4);
+  } else {
+    const __half2 v = __floats2half2_rn(x0, x1);
+    memcpy(&r, &v, 4);
+  }
+  return r;
+}
+
 // 8 consecutive K elements of one row (16 bytes for 16-bit formats, 32 for
 // tf32) at byte offset `off` of a K-major tile: hi (and lo) parts
 template <int FMT, bool SPLIT>
@@ -115,12 +129,9 @@ __device__ __forceinline__ void store8(uint8_t* hi, uint8_t* lo, uint32_t off, c
     uint32_t h[4], l[4];
 #pragma unroll
     for (int e = 0; e < 4; e++) {
-      const uint32_t h0 = enc<FMT>(x[2 * e]), h1 = enc<FMT>(x[2 * e + 1]);
-      h[e] = h0 | (h1 << 16);
-      if constexpr (SPLIT) {
-        const uint32_t l0 = enc<FMT>(x[2 * e] - dec<FMT>(h0)), l1 = enc<FMT>(x[2 * e + 1] - dec<FMT>(h1));
-        l[e] = l0 | (l1 << 16);
-      }
+      h[e] = enc2<FMT>(x[2 * e], x[2 * e + 1]);
+      if constexpr (SPLIT)
+        l[e] = enc2<FMT>(x[2 * e] - dec<FMT>(h[e] & 0xffffu), x[2 * e + 1] - dec<FMT>(h[e] >> 16));
     }
     *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
     if constexpr (SPLIT) *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
@@ -143,6 +154,16 @@ __device__ __forceinline__ void sincos_reduced(float t, float* s, float* c) {
   __sincosf(r, s, c);
 }
 
+__device__ __forceinline__ void st4(float* p, float x, float y, float z, float w) {
+  *reinterpret_cast<float4*>(p) = make_float4(x, y, z, w);
+}
+// 32 bytes in one store; p is 32-byte aligned
+__device__ __forceinline__ void st8(float* p, const float (&v)[8]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
 struct Bars {
   uint64_t wfull[kGemmMaxNW], wfree[kGemmMaxNW];
   uint64_t kfull[kGemmMaxNK], kfree[kGemmMaxNK];
@@ -162,7 +183,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ Bars bars;
   __shared__ uint32_t s_tmem;
-  __shared__ float s_tilt[256];
+  __shared__ __align__(16) float s_tilt[256];  // zero past the last pixel
   __shared__ int s_poff[256];  // pixel -> (row, column) offset in the phase frame
   __shared__ int s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -179,9 +200,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const int nseq = g.noc * g.nkc;
   const int K1B = g.K1 * ESZ;
 
-  for (int k = tid; k < pp; k += blockDim.x) {
-    s_tilt[k] = a.tilt[k];
+  for (int k = tid; k < 256; k += blockDim.x) {
     const int ii = k / p;
+    s_tilt[k] = k < pp ? a.tilt[k] : 0.f;
     s_poff[k] = ii * a.W + (k - ii * p);
   }
   if (tid == 0) s_abort = 0;
@@ -464,22 +485,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                           const float (&puv)[8]) {
       const int pix0 = g8 * 8;
       float er[8], ei[8];
+      // zero where there is no pixel or no row, as the pupil is; without a
+      // branch per pixel the eight sines and cosines overlap (50 frames of a
+      // 40x40 sensor at split products 73.7 -> 68.9 us)
+      const float4 t0 = *reinterpret_cast<const float4*>(&s_tilt[pix0]);
+      const float4 t1 = *reinterpret_cast<const float4*>(&s_tilt[pix0 + 4]);
+      const float tl[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
 #pragma unroll
       for (int e = 0; e < 8; e++) {
-        const int pix = pix0 + e;
-        er[e] = 0.f;
-        ei[e] = 0.f;
-        if (R.live && pix < pp) {
-          const float t = phv[e] - s_tilt[pix];
-          float sn, cs;
-          if constexpr (SPLIT) {
-            sincosf(t, &sn, &cs);
-          } else {
-            sincos_reduced(t, &sn, &cs);
-          }
-          er[e] = puv[e] * cs;
-          ei[e] = puv[e] * sn;
+        const float t = phv[e] - tl[e];
+        float sn, cs;
+        if constexpr (SPLIT) {
+          sincosf(t, &sn, &cs);
+        } else {
+          sincos_reduced(t, &sn, &cs);
         }
+        er[e] = puv[e] * cs;
+        ei[e] = puv[e] * sn;
       }
       store8<FMT, SPLIT>(Ehi, Elo, kmaj(rf, pix0, ESZ, sboE), er);
       store8<FMT, SPLIT>(Ehi, Elo, kmaj(rf, ppr + pix0, ESZ, sboE), ei);
@@ -569,6 +591,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const float scale = nv.scale;  // exactly 1 when there is nothing to scale
         const float skyv = nv.skyv;
         float* out = a.bimg + (long long)P.frm * a.bimgFrameStride + (long long)i * mm;
+        const bool half = (uintptr_t)out & 16;
         const float* skyA = a.skyArr ? a.skyArr + (long long)i * mm : nullptr;
         for (int cb = h * 32; cb < mm && liveLanes; cb += 64) {
           uint32_t v[32];
@@ -584,10 +607,34 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             if (skyv > 0.f) x[e] += skyv;
             if (skyA && e < n) x[e] += skyA[cb + e];
           }
-          if (vecOut) {  // n is a multiple of 4 here
+          if (vecOut) {
+            // n is a multiple of 4 here and rows are 16-byte aligned: whole
+            // 32-byte sectors, from the second four values on in a row that
+            // starts in the middle of one.  With 16-byte stores, a row per
+            // lane, this read-out held the epilogue for 6 of 24 thousand
+            // cycles a tile (64 frames of the 74x74 sensor 335 -> 329 us).
+            float* q = out + cb;
+            if (half && n >= 4) st4(q, x[0], x[1], x[2], x[3]);
 #pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              if (e < n) *reinterpret_cast<float4*>(out + cb + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
+            for (int e = 0; e < 24; e += 8) {
+              const int c = half ? e + 4 : e;
+              float y[8];
+#pragma unroll
+              for (int k = 0; k < 8; k++) y[k] = half ? x[e + 4 + k] : x[e + k];
+              if (c + 8 <= n) {
+                st8(q + c, y);
+              } else if (c + 4 <= n) {
+                st4(q + c, y[0], y[1], y[2], y[3]);
+              }
+            }
+            if (half) {
+              if (n == 32) st4(q + 28, x[28], x[29], x[30], x[31]);
+            } else if (n == 32) {
+              const float y[8] = {x[24], x[25], x[26], x[27], x[28], x[29], x[30], x[31]};
+              st8(q + 24, y);
+            } else if (n == 28) {
+              st4(q + 24, x[24], x[25], x[26], x[27]);
+            }
           } else {
 #pragma unroll
             for (int e = 0; e < 32; e++)

@@ -36,3 +36,29 @@ def test_small_launches_equal_large_ones(form, nsubx, p, N):
         np.testing.assert_array_equal(ce, res[0][0])
     assert np.isfinite(res[0][1]).all() and res[0][1].max() > 0
     eng.free()
+
+
+@pytest.mark.parametrize("m", [2, 4, 5, 6, 8, 10, 12, 14, 16])
+def test_image_rows_at_any_alignment(m):
+    # images stored in whole 32-byte sectors from a 32- or 16-byte aligned
+    # start, and value by value from any other, for every remainder of a row
+    c = Case(nsubx=7, p=8, N=16, C=16, m=m, ncen=m, psf="gauss", sig=1e3, skybrightness=4.0, L0=1.0, obs=0.1)
+    eng = c.engine()
+    eng.set_form("fp16")
+    assert eng.info()["form_active"] != 0
+    frames, size = 3, c.nsubaps * m * m
+    phs = torch.stack([torch.from_numpy(c.new_phase(k)).cuda() for k in range(frames)]).contiguous()
+    res = []
+    for shift in (0, 4, 1):
+        ce = torch.zeros((frames, c.nsubaps * 2), device="cuda")
+        flat = torch.full((frames * size + 8,), -1.0, device="cuda")
+        bi = flat[shift:shift + frames * size].view(frames, c.nsubaps, m, m)
+        eng.run_batch(phs, ce, bi)
+        torch.cuda.synchronize()
+        assert (flat[:shift] == -1).all() and (flat[shift + frames * size:] == -1).all()
+        res.append((bi.cpu().numpy(), ce.cpu().numpy()))
+    for bi, ce in res[1:]:
+        np.testing.assert_array_equal(bi, res[0][0])
+        np.testing.assert_array_equal(ce, res[0][1])
+    assert np.isfinite(res[0][0]).all() and res[0][0].max() > 0
+    eng.free()

@@ -458,16 +458,26 @@ bool corr_active(const shwfs_handle* h) {
   return h->correlationCentroiding != 0 && !h->corrPatHost.empty() && h->imageOnly == 0 && h->opticalBinning != 1;
 }
 
+// the cosines and sines of 2 pi j k / n for one size of hc2r_2d
+struct Hc2rTables {
+  int n;
+  std::vector<double> cs, sn;
+  explicit Hc2rTables(int n_) : n(n_), cs((size_t)n_ * n_), sn((size_t)n_ * n_) {
+    for (int j = 0; j < n; j++)
+      for (int k = 0; k < n; k++) {
+        const double a = 2.0 * M_PI * (double)((long long)j * k % n) / n;
+        cs[(size_t)j * n + k] = cos(a);
+        sn[(size_t)j * n + k] = sin(a);
+      }
+  }
+};
+
 // hc2r x hc2r (FFTW's unnormalised half-complex inverse along each axis) of
 // an n x n half-complex array, in double
-void hc2r_2d(const float* h, int n, std::vector<double>& out) {
-  std::vector<double> cs(n * n), sn(n * n), t((size_t)n * n);
-  for (int j = 0; j < n; j++)
-    for (int k = 0; k < n; k++) {
-      const double a = 2.0 * M_PI * (double)((long long)j * k % n) / n;
-      cs[j * n + k] = cos(a);
-      sn[j * n + k] = sin(a);
-    }
+void hc2r_2d(const float* h, const Hc2rTables& tab, std::vector<double>& out) {
+  const int n = tab.n;
+  const double *cs = tab.cs.data(), *sn = tab.sn.data();
+  std::vector<double> t((size_t)n * n);
   auto line = [&](const double* in, double* o, int stride) {  // one 1-D inverse
     for (int j = 0; j < n; j++) {
       double y = in[0];
@@ -511,9 +521,12 @@ shwfs_status prepare_corr(shwfs_handle* h) {
   const int n = h->corrPatternSize, cc = n * n;
   std::vector<float> K(h->corrPatHost.size());
   if (h->correlationCentroiding == 1) {
+    // one set of tables for all patterns: built for each, they took half of the
+    // first frame (74x74 subapertures, corrsize 20: 46 ms, now 26)
+    const Hc2rTables tab(n);
     std::vector<double> o;
     for (int i = 0; i < h->nsubaps; i++) {
-      hc2r_2d(h->corrPatHost.data() + (size_t)i * cc, n, o);
+      hc2r_2d(h->corrPatHost.data() + (size_t)i * cc, tab, o);
       for (int k = 0; k < cc; k++) K[(size_t)i * cc + k] = (float)o[k];
     }
   } else {
@@ -1996,7 +2009,7 @@ shwfs_status shwfs_test_correlation(int n, const float* img, float* corr) {
   const size_t nn = (size_t)n * n;
   // the pattern's unnormalised inverse transform, as load_corr_pattern
   std::vector<double> k;
-  hc2r_2d(corr, n, k);
+  hc2r_2d(corr, Hc2rTables(n), k);
   std::vector<float> kf(nn);
   for (size_t i = 0; i < nn; i++) kf[i] = (float)k[i];
   float *dImg = nullptr, *dK = nullptr, *dOut = nullptr;

@@ -5,8 +5,8 @@ The reference serves several WFSs of a simulation by giving each its own
 ``science/wfscent.py`` (resource sharing, science/wfscent.py:585-598).  A
 :class:`WfsBatch` captures one readout frame of every handle into a CUDA graph,
 each handle's kernels on their own branch so that sensors of different sizes
-share the GPU (optionally, handles on the FP32 form that share a kernel
-instantiation as one persistent multi-handle kernel), and replays it with
+share the GPU (optionally, handles on the FP32 warp form that share a
+kernel instantiation as one multi-handle kernel), and replays it with
 one launch per frame.  Every handle must
 have its ``phs``, ``cents`` and ``bimg`` bound to CUDA tensors (``set_io``);
 the noise frame index of each handle advances on the device between replays,
@@ -23,7 +23,7 @@ from ._lib import check
 
 class WfsBatch:
     def __init__(self, engines, multi=False):
-        """``multi``: run the FP32-form handles that share a kernel
+        """``multi``: run the handles on the FP32 warp form that share a kernel
         instantiation as one persistent multi-handle kernel (see
         :meth:`set_multi`)."""
         self.engines = list(engines)
@@ -37,8 +37,8 @@ class WfsBatch:
             self.set_multi(True)
 
     def set_multi(self, on=True):
-        """Group FP32-form handles of one kernel instantiation and shared-memory
-        footprint into persistent multi-handle kernel launches (off by
+        """Group handles on the FP32 warp form of one kernel instantiation and
+        shared-memory footprint into persistent multi-handle kernel launches (off by
         default: concurrent per-handle launches measured as fast or faster);
         results are identical either way.  Re-captures the graph."""
         check(_lib.lib().shwfs_batch_set_multi(self._b, 1 if on else 0), "batch_set_multi")
@@ -51,9 +51,9 @@ class WfsBatch:
         check(_lib.lib().shwfs_batch_run(self._b, s), "batch_run")
 
     def multi_launches(self) -> int:
-        """Multi-handle fused-kernel launches in the captured graph: handles on
-        the FP32 form that share a kernel instantiation run as one persistent
-        kernel over all their tiles."""
+        """Multi-handle formation launches in the captured graph: handles on
+        the FP32 warp form that share a kernel instantiation run as one
+        persistent kernel over all their groups."""
         n = ctypes.c_int(0)
         check(_lib.lib().shwfs_batch_multi_launches(self._b, ctypes.byref(n)), "batch_multi_launches")
         return n.value

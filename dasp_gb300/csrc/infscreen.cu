@@ -59,7 +59,7 @@ __device__ __forceinline__ double to_double(float x) {
 // between lines) and by the FP64 rate (3 len^2 multiply-adds at about two a
 // cycle and SM: 2.6 us for 741 elements); a warp per element with its z
 // gathered by modulo from the circular buffer took 35 us for 741.  Here a
-// thread has all its 18 matrix elements of a chunk in flight before the
+// thread has all its 36 matrix elements of a chunk in flight before the
 // vectors are staged in shared memory, and the line's normals, B n and the
 // matrix loads, which do not depend on the line before, run ahead of
 // griddepcontrol.wait: successive lines are launched programmatically and
